@@ -6,9 +6,10 @@
 // stage of the step (fluid_simulation_dcgrid.cu:263-346 order) as one launch
 // over all members: the members' device descriptors travel in the kernel
 // parameters, and a CTA picks its member from the cumulative CTA counts.
-// The pressure cascade is one cooperative launch per round over the members'
-// concatenated cells of one level; p, p~ and div of all members are slices of
-// three batch arenas so the solve addresses them with one base pointer. The
+// The pressure cascade solves small levels of all members on chip, one cluster
+// per member (k_cascade.cu), larger ones by one cooperative launch over the
+// members' concatenated cells; p, p~ and div of all members are slices of
+// three batch arenas so that solve addresses them with one base pointer. The
 // adaptation (scores, radix sorts, selections, moves, refinements, neighbour
 // rebuild, propagation) is likewise one launch per adaptation kernel over all
 // members, each member's sorts and counters kept separate. Per-member arithmetic is the
@@ -37,18 +38,12 @@ struct dcg_batch {
   int planes = 0;
   uint32_t *binfo = nullptr;  // block descriptions of a cascade round, BI_WORDS words per block
   uint32_t *bar = nullptr, *errw = nullptr;
-  // concurrent cascades (solve_barrier bit 2): members with two different level
-  // counts solved by two cooperative launch chains on parallel graph branches,
-  // each with its own barrier words and block-description table
-  std::vector<int> lgroup[2];
-  uint32_t *bar2 = nullptr, *binfo2 = nullptr;
-  cudaStream_t aux = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  int cl_size = 0;  // cluster size of the small levels' solve (0: none)
   std::vector<unsigned long long> arena_off;
   unsigned long long arena_cells = 0;
   float *emis_arena = nullptr;  // members' emission maps, consecutive in member order
   size_t emis_floats = 0;
-  int maxtop = 0, iters = 0;
+  int iters = 0;
   dcg_tuning tune{};
   int solve_grid = 0;
   std::map<int, cudaGraphExec_t> graphs;
@@ -86,9 +81,6 @@ struct dcg_batch {
     for (dcg_sim *s : m) delete s;
     for (void *p : allocs) cudaFree(p);
     if (stage) cudaFreeHost(stage);
-    if (aux) cudaStreamDestroy(aux);
-    if (ev_fork) cudaEventDestroy(ev_fork);
-    if (ev_join) cudaEventDestroy(ev_join);
     if (own_stream && stream) cudaStreamDestroy(stream);
   }
 
@@ -97,8 +89,7 @@ struct dcg_batch {
 
   int set_solve_config() {
     if (tune.solve_barrier < 0 || tune.solve_barrier > 7)
-      return fail(DCG_E_INVALID, "solve_barrier must be 0..7 (bit 0 two-level barrier, bit 1 coarsest-aligned rounds, "
-                                 "bit 2 concurrent cascades of the two level counts)");
+      return fail(DCG_E_INVALID, "solve_barrier must be 0..7 (bit 0: two-level barrier)");
     if (!solve_variant_valid(tune.solve_cache))
       return fail(DCG_E_INVALID, "solve_cache must be 0, 3, 4, 8 or a pipelined variant 16, 18, 19, 32, 34, 35, 64, 66, 83");
     for (int k = 0; k < 4; k++)
@@ -167,25 +158,6 @@ struct dcg_batch {
         launch_restrict_batch(P, st);
       }
   }
-  // the arenas of the planes the cascade runs on; with the correction planes,
-  // the members' descriptors name them too (the prolongation and the cached
-  // alpha * div read them through the descriptor)
-  void bind_planes(SolveBatch &P) const {
-    if (planes == 0) {
-      P.p = p_arena;
-      P.pt = pt_arena;
-      P.div = div_arena;
-      return;
-    }
-    P.p = e_arena;
-    P.pt = et_arena;
-    P.div = rr_arena;
-    for (int i = 0; i < P.n; i++) {
-      P.d[i].p = P.d[i].e;
-      P.d[i].pt = P.d[i].et;
-      P.d[i].div = P.d[i].rr;
-    }
-  }
   // FP64 defect correction after the cascade (dcg_sim::defect_correct for
   // every member): per pass the FP64 residual and norms, the cascade on the
   // residual into e, and p += e; a last residual measures the result
@@ -212,76 +184,57 @@ struct dcg_batch {
       }
     }
   }
-  // the cascade with the tuned schedule of each round
-  bool can_split() const { return n() <= BMAX && !lgroup[0].empty() && !lgroup[1].empty() && aux; }
-  // one member group's whole cascade (all its members have the same level count)
-  void solve_group(int gi, int grid, int cache, int tree, cudaStream_t st) {
-    const std::vector<int> &mem = lgroup[gi];
-    const int top = m[mem[0]]->D.g.levels - 1;
-    for (int round = 0; round <= top; round++) {
-      SolveBatch P{};
-      P.n = (int)mem.size();
-      P.maxtop = top;
-      P.prolong = 1;
-      P.binfo = gi ? binfo2 : binfo;
-      P.bar = gi ? bar2 : bar;
-      P.err = errw;
-      for (int i = 0; i < P.n; i++) {
-        P.d[i] = m[mem[i]]->D;
-        P.arena[i] = arena_off[mem[i]];
-      }
-      bind_planes(P);
-      launch_level_solve_batch(P, round, iters, grid, cache, tree & 1, st);
-    }
-  }
-  void solve_split(int grid, int cache, int tree) {
-    cudaEventRecord(ev_fork, stream);
-    cudaStreamWaitEvent(aux, ev_fork, 0);
-    solve_group(0, grid, cache, tree, stream);
-    solve_group(1, grid, cache, tree, aux);
-    cudaEventRecord(ev_join, aux);
-    cudaStreamWaitEvent(stream, ev_join, 0);
-  }
+  // the cascade with the tuned schedule of each round of the general solve
   void solve_tuned() {
-    if ((tune.solve_barrier & 4) && can_split()) {
-      solve_split(solve_grid, tune.solve_cache, tune.solve_barrier);
-      return;
-    }
-    for (int round = 0; round <= maxtop; round++) {
-      if (round < 4 && tune.round_ctas_per_sm[round] != 0)
-        solve_round(round, batch_solve_grid(sms, tune.round_cache[round], tune.round_ctas_per_sm[round]),
-                    tune.round_cache[round], tune.round_barrier[round]);
-      else
-        solve_round(round, solve_grid, tune.solve_cache, tune.solve_barrier & 1);
-    }
+    solve([&](int round, int &grid, int &cache, int &tree) {
+      if (round < 4 && tune.round_ctas_per_sm[round] != 0) {
+        cache = tune.round_cache[round];
+        grid = batch_solve_grid(sms, cache, tune.round_ctas_per_sm[round]);
+        tree = tune.round_barrier[round];
+      } else {
+        grid = solve_grid;
+        cache = tune.solve_cache;
+        tree = tune.solve_barrier & 1;
+      }
+    });
   }
-  void solve(int grid, int cache, int tree) {
-    if ((tune.solve_barrier & 4) && can_split()) {
-      solve_split(grid, cache, tree);
-      return;
+  template <class Schedule> void solve(Schedule schedule) {
+    std::vector<Dev> d(n());
+    for (int i = 0; i < n(); i++) {
+      d[i] = m[i]->D;
+      if (planes) {  // the prolongation and the cached alpha * div read these through the descriptor
+        d[i].p = d[i].e;
+        d[i].pt = d[i].et;
+        d[i].div = d[i].rr;
+      }
     }
-    for (int round = 0; round <= maxtop; round++) solve_round(round, grid, cache, tree);
-  }
-  // tree: two-level barrier; the round alignment comes from tune.solve_barrier's bit 1
-  void solve_round(int round, int grid, int cache, int tree) {
-    tree = (tree & 1) | (tune.solve_barrier & 2);
-    {
-      for (int g = 0; g < groups(); g++) {
+    Cascade c;
+    c.csize = cl_size;
+    c.sms = sms;
+    c.sweeps = iters;
+    c.st = stream;
+    c.run(d.data(), n(), [&](const std::vector<int> &mem, const std::vector<int> &lev, long long limit, int round) {
+      int grid = 0, cache = 0, tree = 0;
+      schedule(round, grid, cache, tree);
+      for (size_t g = 0; g < mem.size(); g += BMAX) {
         SolveBatch P{};
-        P.n = std::min(BMAX, n() - g * BMAX);
-        P.maxtop = maxtop;
+        P.n = (int)std::min<size_t>(BMAX, mem.size() - g);
         P.prolong = 1;
+        P.p = planes ? e_arena : p_arena;
+        P.pt = planes ? et_arena : pt_arena;
+        P.div = planes ? rr_arena : div_arena;
         P.binfo = binfo;
         P.bar = bar;
         P.err = errw;
         for (int i = 0; i < P.n; i++) {
-          P.d[i] = m[g * BMAX + i]->D;
-          P.arena[i] = arena_off[g * BMAX + i];
+          P.d[i] = d[mem[g + i]];
+          P.arena[i] = arena_off[mem[g + i]];
+          P.lev[i] = lev[g + i];
+          P.cl_max[i] = limit;
         }
-        bind_planes(P);
-        launch_level_solve_batch(P, round, iters, grid, cache, tree, stream);  // bit 1: alignment
+        launch_level_solve_batch(P, iters, grid, cache, tree, stream);
       }
-    }
+    });
   }
   void flip_v() {
     for (dcg_sim *s : m) {
@@ -324,42 +277,6 @@ struct dcg_batch {
       restrict_fields(1);
     }
   }
-  // With rounds aligned at the coarsest levels, the members with fewer levels
-  // finish their cascade a round early. Their pressure application, scalar
-  // advection and restrictions then run on the second stream (a parallel
-  // graph branch) while the last rounds relax the other members: the
-  // stages read and write only their own members' planes, and the late
-  // rounds, small and bound by their grid barriers, leave most of the GPU free.
-  bool overlapped() const {
-    return dpass == 0 && fused() && can_split() && (tune.solve_barrier & 2) && !(tune.solve_barrier & 4);
-  }
-  void apply_advect_members(const std::vector<int> &mem, cudaStream_t st) {
-    cells(5, mem, st);  // apply pressure + advect scalars (+ sources, emission)
-    for (int i : mem) {
-      m[i]->qpar ^= 1;
-      m[i]->bind_parity();
-    }
-    restrict_fields(3, mem, st);
-  }
-  void solve_apply_overlapped() {
-    const int ga = m[lgroup[0][0]]->D.g.levels < m[lgroup[1][0]]->D.g.levels ? 0 : 1;  // fewer levels
-    const int last = m[lgroup[ga][0]]->D.g.levels - 1;  // its last round
-    for (int round = 0; round <= maxtop; round++) {
-      if (round < 4 && tune.round_ctas_per_sm[round] != 0)
-        solve_round(round, batch_solve_grid(sms, tune.round_cache[round], tune.round_ctas_per_sm[round]),
-                    tune.round_cache[round], tune.round_barrier[round]);
-      else
-        solve_round(round, solve_grid, tune.solve_cache, tune.solve_barrier & 1);
-      if (round == last) {
-        cudaEventRecord(ev_fork, stream);
-        cudaStreamWaitEvent(aux, ev_fork, 0);
-        apply_advect_members(lgroup[ga], aux);
-        cudaEventRecord(ev_join, aux);
-      }
-    }
-    apply_advect_members(lgroup[1 - ga], stream);
-    cudaStreamWaitEvent(stream, ev_join, 0);
-  }
   void step_once() {
     cells(0);  // advect velocity (+ buoyancy)
     flip_v();
@@ -367,10 +284,6 @@ struct dcg_batch {
     adapt();
     cells(2);  // divergence
     restrict_fields(2);
-    if (overlapped()) {
-      solve_apply_overlapped();
-      return;
-    }
     solve_tuned();
     if (dpass > 0) defect_correct();
     apply_advect();
@@ -456,7 +369,6 @@ struct dcg_batch {
     int rc;
     if ((rc = cuda(cudaStreamSynchronize(stream), "sync"))) return rc;
     cudaMemsetAsync(bar, 0, 4 * (64 + 32 * 18), stream);
-    if (bar2) cudaMemsetAsync(bar2, 0, 4 * (64 + 32 * 18), stream);
     cudaMemsetAsync(errw, 0, 4, stream);
     for (dcg_sim *s : m)
       if ((rc = s->reset_adaptive())) return fail(rc, "member reset: " + s->err);
@@ -546,17 +458,22 @@ struct dcg_batch {
       best.tile[stage] = tune.tile[stage] = tile_of[pick][stage];
       best.cells_ms[stage] = ms_of[pick][stage];
     }
-    // level solve: cache depth x CTAs per SM x barrier kind
+    // the general level solve (levels that no cluster holds): cache depth x
+    // CTAs per SM x barrier kind, timed with the whole cascade
     float best_solve = 1e30f;
+    for (int r = 0; r < 4; r++) best.round_ctas_per_sm[r] = 0;
     for (int cache : {0, 3, 4, 8, 16, 18, 19, 32, 34, 35, 64, 66, 83}) {
       const int occ = batch_solve_grid(sms, cache, 0) / std::max(1, sms);
       for (int k = 1; k <= occ; k++)
-        for (int tb = 0; tb < 8; tb++) {  // bit 0: two-level barrier; bit 1: coarsest-aligned rounds;
-                                          // bit 2: concurrent cascades per level count
-          if ((tb & 4) && (!can_split() || (tb & 2))) continue;
-          tune.solve_barrier = tb;
+        for (int tb = 0; tb < 2; tb++) {  // two-level barrier
           const int grid = batch_solve_grid(sms, cache, k);
-          const float ms = time_ms(reps, [&] { solve(grid, cache, tb & 1); });
+          const float ms = time_ms(reps, [&] {
+            solve([&](int, int &g, int &c, int &t) {
+              g = grid;
+              c = cache;
+              t = tb;
+            });
+          });
           if (ms < best_solve) {
             best_solve = ms;
             best.solve_cache = cache;
@@ -564,34 +481,6 @@ struct dcg_batch {
             best.solve_barrier = tb;
           }
         }
-    }
-    tune.solve_barrier = best.solve_barrier;  // the per-round schedules below use its alignment
-    // each round of the first four on its own: the best schedule if it beats
-    // the whole-cascade choice for that round (not with concurrent cascades)
-    for (int r = 0; r < 4 && r <= maxtop && !(best.solve_barrier & 4); r++) {
-      const float base = time_ms(reps, [&] {
-        solve_round(r, batch_solve_grid(sms, best.solve_cache, best.solve_ctas_per_sm), best.solve_cache,
-                    best.solve_barrier);
-      });
-      float bms = base;
-      best.round_ctas_per_sm[r] = 0;
-      for (int cache : {0, 3, 4, 8, 16, 18, 19, 32, 34, 35, 64, 66, 83}) {
-        const int occ = batch_solve_grid(sms, cache, 0) / std::max(1, sms);
-        std::vector<int> ks = {-8, -4, -2};  // k < 0: one CTA per -k SMs (small rounds)
-        for (int k = 1; k <= occ; k++) ks.push_back(k);
-        for (int k : ks)
-          for (int tree = 0; tree < 2; tree++) {
-            const int grid = batch_solve_grid(sms, cache, k);
-            const float ms = time_ms(reps, [&] { solve_round(r, grid, cache, tree); });
-            if (ms < 0.97f * bms) {
-              bms = ms;
-              best.round_ctas_per_sm[r] = (int16_t)k;
-              best.round_cache[r] = (int8_t)cache;
-              best.round_barrier[r] = (int8_t)tree;
-            }
-          }
-      }
-      best_solve += bms - base;
     }
     best.solve_ms = best_solve;
     if ((rc = sync())) return rc;
@@ -720,11 +609,6 @@ int dcg_batch_create(int32_t n, const dcg_params *params, dcg_batch **out) {
     delete b;
     return rc;
   }
-  if ((rc = b->alloc(&b->bar2, 64 + 32 * 18)) || (rc = b->alloc(&b->binfo2, BI_WORDS * (cells / BV)))) {
-    delete b;
-    return rc;
-  }
-  cudaMemset(b->bar2, 0, 4 * (64 + 32 * 18));
   cudaMemset(b->errw, 0, 4);
   size_t emis_at = 0;
   for (int i = 0; i < n; i++) {
@@ -755,7 +639,6 @@ int dcg_batch_create(int32_t n, const dcg_params *params, dcg_batch **out) {
       delete b;
       return rc;
     }
-    b->maxtop = std::max(b->maxtop, s->D.g.levels - 1);
     SortScratch S2{};
     const long long nb = s->D.g.B, nt = sort_tiles(nb);
     if ((rc = b->alloc(&S2.k1, nb)) || (rc = b->alloc(&S2.v1, nb)) || (rc = b->alloc(&S2.hist, 256 * nt)) ||
@@ -766,26 +649,7 @@ int dcg_batch_create(int32_t n, const dcg_params *params, dcg_batch **out) {
     S2.max_n = nb;
     b->S2.push_back(S2);
   }
-  // level-count groups for concurrent cascades: exactly two level counts
-  {
-    int la = -1, lb = -1;
-    bool two = true;
-    for (int i = 0; i < n; i++) {
-      const int L = b->m[i]->D.g.levels;
-      if (la < 0 || L == la) la = L;
-      else if (lb < 0 || L == lb) lb = L;
-      else two = false;
-    }
-    if (two && lb >= 0) {
-      for (int i = 0; i < n; i++) b->lgroup[b->m[i]->D.g.levels == la ? 0 : 1].push_back(i);
-      if (cudaStreamCreateWithFlags(&b->aux, cudaStreamNonBlocking) != cudaSuccess ||
-          cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
-          cudaEventCreateWithFlags(&b->ev_join, cudaEventDisableTiming) != cudaSuccess) {
-        delete b;
-        return DCG_E_CUDA;
-      }
-    }
-  }
+  b->cl_size = cluster_solve_size();
   for (int k = 0; k < 4; k++) b->tune.tile[k] = 4;
   b->tune.solve_cache = 4;
   b->tune.solve_ctas_per_sm = 0;

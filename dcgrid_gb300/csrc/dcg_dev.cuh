@@ -258,32 +258,56 @@ __device__ inline uint32_t descend(const Dev &D, uint32_t b, int &l, int qx, int
 // x / 6, correctly rounded, by the method for divisors known in advance of
 // Brisebarre, Muller and Raina (IEEE Trans. Computers 53(8), 2004): q =
 // RN(x z) with z = RN(1/6), the remainder x - 6q exactly by one FMA, then
-// RN(q + r z). The method assumes no underflow: inputs below 2^-120 in
-// magnitude (subnormal quotients, signed zeros) take the IEEE division.
-// Infinite x gives a NaN remainder; q (= x / 6 for those) is returned then.
-// The library's self-check (dcg_check_div6) compares the result with the
-// IEEE division over every binary32 input.
+// RN(q + r z). A zero remainder means that q is exact, which keeps the sign
+// of a zero x (most cells far from a source are zero); infinite x gives a
+// NaN remainder, and q is the quotient then too. The method assumes no
+// underflow: nonzero inputs below 2^-120 in magnitude (subnormal quotients)
+// take the IEEE division. The library's self-check (dcg_check_div6) compares
+// the result with the IEEE division over every binary32 input.
 __device__ __forceinline__ float div6(float x) {
-  if (!(fabsf(x) >= 0x1p-120f) && x == x) return x / 6.f;
   const float z = 0x1.555556p-3f;
   const float q = __fmul_rn(x, z);
   const float r = fmaf(-q, 6.f, x);
   const float y = fmaf(r, z, q);
-  return r == r ? y : q;
-}
-
-// div6 of both components with packed FP32x2 operations (each component the
-// correctly rounded operation of div6's scalar form, so the results are div6's)
-__device__ __forceinline__ float2 div6x2(float2 x) {
-  const float2 z = make_float2(0x1.555556p-3f, 0x1.555556p-3f);
-  const float2 q = __fmul2_rn(x, z);
-  const float2 r = __ffma2_rn(q, make_float2(-6.f, -6.f), x);  // x - 6 q, exactly as fmaf(-q, 6, x)
-  const float2 y = __ffma2_rn(r, z, q);
-  float2 o;
-  o.x = (!(fabsf(x.x) >= 0x1p-120f) && x.x == x.x) ? x.x / 6.f : (r.x == r.x ? y.x : q.x);
-  o.y = (!(fabsf(x.y) >= 0x1p-120f) && x.y == x.y) ? x.y / 6.f : (r.y == r.y ? y.y : q.y);
+  float o = fabsf(r) > 0.f ? y : q;
+  if (fabsf(x) < 0x1p-120f && x != 0.f) o = x / 6.f;
   return o;
 }
+
+// div6 of the components of N pairs with packed FP32x2 operations (each
+// component the correctly rounded operation of div6's scalar form, so the
+// results are div6's). One test of the smallest magnitude sends the lane to
+// the component-wise subnormal test, which developed flows rarely need.
+__device__ __noinline__ inline float div6_small(float x) { return x / 6.f; }
+template <int N> __device__ __forceinline__ void div6_pairs(float2 (&x)[N]) {
+  const float2 z = make_float2(0x1.555556p-3f, 0x1.555556p-3f);
+  float2 o[N];
+  float small = fminf(fabsf(x[0].x), fabsf(x[0].y));
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    const float2 q = __fmul2_rn(x[i], z);
+    const float2 r = __ffma2_rn(q, make_float2(-6.f, -6.f), x[i]);  // x - 6 q, exactly as fmaf(-q, 6, x)
+    const float2 y = __ffma2_rn(r, z, q);
+    o[i].x = fabsf(r.x) > 0.f ? y.x : q.x;
+    o[i].y = fabsf(r.y) > 0.f ? y.y : q.y;
+    if (i > 0) small = fminf(small, fminf(fabsf(x[i].x), fabsf(x[i].y)));
+  }
+  if (small < 0x1p-120f) {
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      if (fabsf(x[i].x) < 0x1p-120f && x[i].x != 0.f) o[i].x = div6_small(x[i].x);
+      if (fabsf(x[i].y) < 0x1p-120f && x[i].y != 0.f) o[i].y = div6_small(x[i].y);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < N; i++) x[i] = o[i];
+}
+__device__ __forceinline__ float2 div6x2(float2 x) {
+  float2 v[1] = {x};
+  div6_pairs(v);
+  return v[0];
+}
+__device__ __forceinline__ void div6x8(float2 (&x)[4]) { div6_pairs(x); }
 
 __device__ inline int dir_of(int a) { return a == 0 ? 0 : (a == AW - 1 ? 2 : 1); }
 
@@ -308,6 +332,33 @@ __device__ inline unsigned long long apron_cell(const Dev &D, uint32_t b, int4 b
   const int k = (int)(e >> 28);
   const int cx = bp.x + ax - 1, cy = bp.y + ay - 1, cz = bp.z + az - 1;
   return (unsigned long long)nb * BV + local_of((cx >> k) & 3, (cy >> k) & 3, (cz >> k) & 3);
+}
+
+// Prolongation (k_dcgrid_prolongate, dcgrid_multigrid_solver.cu:43-76) of cell
+// c of block b: the 27/9/3/1 interpolation of D.p from the parent block's
+// apron; `out` is left as it is where the block has no parent. The loads go
+// to L2: the parent's values may have been written inside the same launch.
+__device__ inline void prolong_value(const Dev &D, uint32_t b, int c, float &out) {
+  const uint32_t par = D.parent[b];
+  if (par == NONE) return;
+  const int4 bp = D.pos[b];
+  const uint32_t pb = par >> 3;
+  const int4 pbp = D.pos[pb];
+  int lx, ly, lz;
+  local_xyz(c, lx, ly, lz);
+  const int x = bp.x + lx, y = bp.y + ly, z = bp.z + lz;
+  const int ax = 1 + (x / 2) % BW, ay = 1 + (y / 2) % BW, az = 1 + (z / 2) % BW;
+  const int i = x % 2 ? 1 : -1, j = y % 2 ? 1 : -1, k = z % 2 ? 1 : -1;
+  const float *P = D.p;
+  const float p000 = __ldcg(P + apron_cell(D, pb, pbp, ax, ay, az));
+  const float p001 = __ldcg(P + apron_cell(D, pb, pbp, ax, ay, az + k));
+  const float p010 = __ldcg(P + apron_cell(D, pb, pbp, ax, ay + j, az));
+  const float p100 = __ldcg(P + apron_cell(D, pb, pbp, ax + i, ay, az));
+  const float p011 = __ldcg(P + apron_cell(D, pb, pbp, ax, ay + j, az + k));
+  const float p101 = __ldcg(P + apron_cell(D, pb, pbp, ax + i, ay, az + k));
+  const float p110 = __ldcg(P + apron_cell(D, pb, pbp, ax + i, ay + j, az));
+  const float p111 = __ldcg(P + apron_cell(D, pb, pbp, ax + i, ay + j, az + k));
+  out = (27.f * p000 + 9.f * (p001 + p010 + p100) + 3.f * (p011 + p101 + p110) + p111) / 64.f;
 }
 
 // The six Jacobi neighbours (L, R, D, U, B, F) of a cell, as global cell indices.

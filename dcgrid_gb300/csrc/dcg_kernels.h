@@ -75,18 +75,29 @@ struct RestrictBatch {
   Dev d[BMAX];
   FieldList fl[BMAX];
 };
-// Cascade round r solves level maxtop - r of every member that has it (finest
-// levels aligned); p and p~ of all members are slices of two arenas.
+// One cooperative solve of one level per member: member s's level lev[s] (-1:
+// none) unless the cluster solve takes it (its load is at most cl_max[s]
+// blocks); p and p~ of all members are slices of two arenas.
 struct SolveBatch {
-  int n, maxtop, prolong, pad;
+  int n, prolong;
   float *p, *pt;
   const float *div;  // divergence arena (same layout as p)
   uint32_t *binfo;   // block descriptions of the round's level, BI_WORDS words per level block
   uint32_t *bar, *err;
   unsigned long long arena[BMAX];  // first cell of member s in the arenas
+  int lev[BMAX];
+  long long cl_max[BMAX];
   Dev d[BMAX];
 };
-static_assert(sizeof(RestrictBatch) < 32000 && sizeof(SolveBatch) < 32000, "kernel parameter space");
+// Cluster solve (k_cascade.cu): member s's levels hi[s] down to lo[s], one
+// after the other, those with at most `limit` allocated blocks
+struct ClusterSolve {
+  int n, csize, sweeps, prolong;
+  long long limit;
+  int hi[BMAX], lo[BMAX];
+  Dev d[BMAX];
+};
+static_assert(sizeof(RestrictBatch) < 32000 && sizeof(SolveBatch) < 32000 && sizeof(ClusterSolve) < 32000, "kernel parameter space");
 // persistent: a grid of a few CTAs per SM over the allocated blocks only
 void launch_cells_batch(int stage, CellBatch &P, int tile, cudaStream_t st, bool persistent = false);
 void launch_restrict_batch(RestrictBatch &P, cudaStream_t st);
@@ -108,8 +119,31 @@ void launch_add_correction_batch(CellBatch &P, cudaStream_t st);
 // and CTAs per SM (0 = occupancy limit)
 int batch_solve_grid(int sms, int cache, int ctas_per_sm);
 bool solve_variant_valid(int cache);
-void launch_level_solve_batch(const SolveBatch &P, int round, int sweeps, int grid, int cache, int tree,
-                              cudaStream_t st);
+void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cache, int tree, cudaStream_t st);
+
+// k_cascade.cu: cluster size of the device's cluster solve (0: none), blocks a
+// cluster of that size holds, and the launch (it picks P.csize)
+int cluster_solve_size();
+long long cluster_solve_blocks(int csize);
+void launch_cluster_solve(ClusterSolve &P, int max_csize, long long max_blocks, int sms, cudaStream_t st);
+
+// Host schedule of a cascade over any number of simulations: every level of
+// every member, coarse to fine, each by the solver that suits it. The levels
+// whose budget a cluster holds go to the cluster solve, runs of them in one
+// launch; a larger level goes there too while its allocated blocks fit
+// (known on the device only), else to `general`, which is launched behind it
+// and leaves what the cluster solve took.
+struct Cascade {
+  int csize = 0;  // cluster size of the device (0: no cluster solve)
+  int sms = 148;
+  int sweeps = 0, prolong = 1;
+  cudaStream_t st = nullptr;
+  long long limit() const { return csize > 0 ? cluster_solve_blocks(csize) : 0; }
+  // general(members, levels, limit, round): solve levels[i] of members[i]
+  // unless at most `limit` of its blocks are allocated
+  // only >= 0: that level alone
+  template <class General> void run(const Dev *d, int n, General general, int only = -1) const;
+};
 
 // self-check of the solver's division by six: bad[0] += mismatches, bad[1] = min mismatching input
 void launch_check_div6(unsigned long long *bad, int sms, cudaStream_t st);

@@ -25,6 +25,65 @@ int idiv_up(int a, int b) { return (a % b != 0) ? (a / b + 1) : (a / b); }
 
 }  // namespace
 
+namespace dcg {
+template <class General> void Cascade::run(const Dev *d, int n, General general, int only) const {
+  // The grid-wide solve shares its barriers over the members of a round, the
+  // clusters share nothing: a batch with more blocks than clusters hold at once
+  // stays with it (16 plumes of 64^3 to 256^3: 9.9 ms per step, 11.6 ms with
+  // clusters; 10 plumes of 32^3 to 64^3: 0.54 ms, 0.41 ms with clusters).
+  long long lim = limit(), all = 0;
+  for (int i = 0; i < n; i++)
+    for (int l = 0; l < d[i].g.levels; l++) all += d[i].g.budget[l];
+  if (n > 1 && all > 8 * lim) lim = 0;
+  std::vector<int> cur(n);
+  for (int i = 0; i < n; i++) cur[i] = only >= 0 ? only : d[i].g.levels - 1;
+  const int last = only >= 0 ? only : 0;
+  for (int round = 0;; round++) {
+    std::vector<int> mem, hi, lo, gm, gl;  // cluster runs; members and levels left to `general`
+    long long blocks = 0;
+    bool left = false;
+    for (int i = 0; i < n; i++) {
+      if (cur[i] < last) continue;
+      left = true;
+      const Geom &g = d[i].g;
+      const int top = cur[i];
+      int l = top;
+      while (l >= last && g.budget[l] <= lim) blocks = std::max(blocks, g.budget[l--]);
+      if (l >= last) {
+        if (lim > 0 && g.budget[l] < g.full[l]) blocks = lim;
+        gm.push_back(i);
+        gl.push_back(l);
+        cur[i] = l - 1;
+        if (!(lim > 0 && g.budget[l] < g.full[l])) l++;  // allocated in full: never fits
+      } else {
+        cur[i] = -1;
+        l = last;
+      }
+      if (l <= top) {
+        mem.push_back(i);
+        hi.push_back(top);
+        lo.push_back(l);
+      }
+    }
+    if (!left) return;
+    for (size_t g = 0; g < mem.size(); g += BMAX) {
+      ClusterSolve P{};
+      P.n = (int)std::min<size_t>(BMAX, mem.size() - g);
+      P.sweeps = sweeps;
+      P.prolong = prolong;
+      P.limit = lim;
+      for (int i = 0; i < P.n; i++) {
+        P.d[i] = d[mem[g + i]];
+        P.hi[i] = hi[g + i];
+        P.lo[i] = lo[g + i];
+      }
+      launch_cluster_solve(P, csize, blocks, sms, st);
+    }
+    if (!gm.empty()) general(gm, gl, lim, round);
+  }
+}
+}  // namespace dcg
+
 struct dcg_sim {
   dcg_params P{};
   int mode = DCG_MODE_ADAPTIVE;
@@ -74,6 +133,7 @@ struct dcg_sim {
   // the staged solve's cooperative grid cannot be formed on the device
   int ls_epoch = 3;
   int ls_grid_staged = 0;  // CTAs of the staged solve
+  int cl_size = 0;         // cluster size of the small levels' solve (0: none)
   // level solve of single simulations: pipelined staged sweeps, two tile buffers,
   // block descriptions cached in 3 x 8 KB of shared memory when they fit.
   // Variant 19 (3 CTAs per SM, two blocks per claim); variant 83 (4 CTAs per
@@ -315,6 +375,7 @@ struct dcg_sim {
     ls_grid = level_solve_grid(sms);
     ls_grid_staged = batch_solve_grid(sms, kSolveVariant, 0);
     if (ls_grid_staged <= 0 && ls_epoch == 3) ls_epoch = 2;
+    cl_size = cluster_solve_size();
     if (P.emission_n > 0) {
       const size_t ne = (size_t)P.emission_n * P.emission_n * P.emission_n;
       if (ext_emis) emis = ext_emis;
@@ -437,7 +498,7 @@ struct dcg_sim {
       // level, nor in projectLocal) and all of the level's sweeps
       const int sweeps = local ? 2 * P.jacobi_iters : P.jacobi_iters;
       if (ls_epoch == 3) {
-        for (int l = top; l >= 0; l--) solve_staged(l, local ? 0 : 1, sweeps);
+        solve_cascade(local ? 0 : 1, sweeps);
         if (!local && P.defect_passes > 0) defect_correct(sweeps);
       } else {
         for (int l = top; l >= 0; l--)
@@ -496,7 +557,7 @@ struct dcg_sim {
   // every level's equations (norms into dnorm), the cascade on the residual
   // into e, and p += e; a last residual measures the result
   void defect_correct(int sweeps) {
-    const int K = P.defect_passes, top = D.g.levels - 1;
+    const int K = P.defect_passes;
     cudaMemsetAsync(D.dnorm, 0, sizeof(double) * 2 * (K + 1), stream);
     for (int k = 0; k <= K; k++) {
       CellBatch C{};  // the staged FP64 residual of pass k
@@ -506,34 +567,58 @@ struct dcg_sim {
       launch_cells_batch(6, C, 1, stream);
       if (k == K) break;
       cudaMemsetAsync(D.e, 0, (size_t)D.g.B * BV * sizeof(float), stream);
-      for (int l = top; l >= 0; l--) solve_staged(l, 1, sweeps, D.e, D.et, D.rr);
+      solve_cascade(1, sweeps, D.e, D.et, D.rr);
       launch_add_correction(D, stream);
     }
   }
 
-  // one level of the cascade through the staged solve, as a batch of one
-  // (prolongation only below the coarsest level), on p / p~ / div or on the
-  // given planes
-  void solve_staged(int level, int prolong, int sweeps, float *pp = nullptr, float *ppt = nullptr,
-                    float *pdiv = nullptr) {
+  // the whole cascade on p / p~ / div, or on the given planes
+  void solve_cascade(int prolong, int sweeps, float *pp = nullptr, float *ppt = nullptr, float *pdiv = nullptr) {
+    Dev d = D;
+    if (pp) {
+      d.p = pp;
+      d.pt = ppt;
+      d.div = pdiv;
+    }
+    Cascade c;
+    c.csize = cl_size;
+    c.sms = sms;
+    c.sweeps = sweeps;
+    c.prolong = prolong;
+    c.st = stream;
+    c.run(&d, 1, [&](const std::vector<int> &, const std::vector<int> &lev, long long limit, int) {
+      solve_staged(d, lev[0], prolong, sweeps, limit);
+    });
+  }
+  // one level on its own, without prolongation (measurements)
+  void solve_level(int level, int sweeps) {
+    Cascade c;
+    c.csize = cl_size;
+    c.sms = sms;
+    c.sweeps = sweeps;
+    c.prolong = 0;
+    c.st = stream;
+    c.run(&D, 1, [&](const std::vector<int> &, const std::vector<int> &lev, long long limit, int) {
+      solve_staged(D, lev[0], 0, sweeps, limit);
+    }, level);
+  }
+  // one level through the staged solve, as a batch of one (prolongation only
+  // below the coarsest level), unless at most `limit` blocks are allocated
+  void solve_staged(const Dev &d, int level, int prolong, int sweeps, long long limit) {
     SolveBatch SB{};
     SB.n = 1;
-    SB.maxtop = D.g.levels - 1;
     SB.prolong = prolong;
-    SB.p = pp ? pp : D.p;
-    SB.pt = ppt ? ppt : D.pt;
-    SB.div = pdiv ? pdiv : D.div;
+    SB.p = d.p;
+    SB.pt = d.pt;
+    SB.div = d.div;
     SB.binfo = D.binfo;
     SB.bar = D.bar;
     SB.err = D.err;
     SB.arena[0] = 0;
-    SB.d[0] = D;
-    if (pp) {  // the prolongation and the cached alpha*div read these through D
-      SB.d[0].p = pp;
-      SB.d[0].pt = ppt;
-      SB.d[0].div = pdiv;
-    }
-    launch_level_solve_batch(SB, SB.maxtop - level, sweeps, ls_grid_staged, kSolveVariant, 1, stream);
+    SB.lev[0] = level;
+    SB.cl_max[0] = limit;
+    SB.d[0] = d;
+    launch_level_solve_batch(SB, sweeps, ls_grid_staged, kSolveVariant, 1, stream);
   }
   void a_advect_scalars() {
     cells(1, 1);

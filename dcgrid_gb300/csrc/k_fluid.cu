@@ -291,27 +291,11 @@ __global__ void __launch_bounds__(256) k_prolongate(Dev D, int level) {
 
 // One cell of k_prolongate, addressed by its global cell index.
 __device__ inline void prolong_cell(const Dev &D, long long cell) {
+  float v = 0.f;
   const uint32_t b = (uint32_t)(cell >> 6);
-  const uint32_t par = D.parent[b];
-  if (par == NONE) return;
-  const int4 bp = D.pos[b];
-  const uint32_t pb = par >> 3;
-  const int4 pbp = D.pos[pb];
-  int lx, ly, lz;
-  local_xyz((int)(cell & 63), lx, ly, lz);
-  const int x = bp.x + lx, y = bp.y + ly, z = bp.z + lz;
-  const int ax = 1 + (x / 2) % BW, ay = 1 + (y / 2) % BW, az = 1 + (z / 2) % BW;
-  const int i = x % 2 ? 1 : -1, j = y % 2 ? 1 : -1, k = z % 2 ? 1 : -1;
-  const float *P = D.p;
-  const float p000 = P[apron_cell(D, pb, pbp, ax, ay, az)];
-  const float p001 = P[apron_cell(D, pb, pbp, ax, ay, az + k)];
-  const float p010 = P[apron_cell(D, pb, pbp, ax, ay + j, az)];
-  const float p100 = P[apron_cell(D, pb, pbp, ax + i, ay, az)];
-  const float p011 = P[apron_cell(D, pb, pbp, ax, ay + j, az + k)];
-  const float p101 = P[apron_cell(D, pb, pbp, ax + i, ay, az + k)];
-  const float p110 = P[apron_cell(D, pb, pbp, ax + i, ay + j, az)];
-  const float p111 = P[apron_cell(D, pb, pbp, ax + i, ay + j, az + k)];
-  D.p[cell] = (27.f * p000 + 9.f * (p001 + p010 + p100) + 3.f * (p011 + p101 + p110) + p111) / 64.f;
+  if (D.parent[b] == NONE) return;
+  prolong_value(D, b, (int)(cell & 63), v);
+  D.p[cell] = v;
 }
 
 // Loads go through L2 (__ldcg): inside one persistent launch the ping-pong
@@ -981,9 +965,10 @@ __device__ __forceinline__ void solve_pipelined(const SolveBatch &P, const long 
   }
 }
 
-// One round of the batched cascade: level maxtop - round of every member that
-// has it, optional prolongation from the member's parent level, then `sweeps`
-// Jacobi sweeps over the concatenated cells of all members, separated by grid
+// One round of the batched cascade: level P.lev[m] of every member m that has
+// one and whose level the cluster solve leaves (more than P.cl_max[m] blocks),
+// optional prolongation from the member's parent level, then `sweeps` Jacobi
+// sweeps over the concatenated cells of all members, separated by grid
 // barriers (tree & 1: two-level barrier). Member m's cells of the level
 // occupy [s_end[m-1], s_end[m]) of the concatenated index. With CACHE > 0 and
 // at most CACHE cells per thread, each thread keeps, per cell, the six
@@ -994,7 +979,7 @@ __device__ __forceinline__ void solve_pipelined(const SolveBatch &P, const long 
 // of k_jacobi (identical results).
 template <int CACHE, int NB = 0, int MB = DCG_PIPE_MINB, int CLAIM = DCG_PIPE_CLAIM>
 __global__ void __launch_bounds__(256, NB ? MB : DCG_SOLVE_MINB)
-    k_level_solve_batch(const __grid_constant__ SolveBatch P, int round, int sweeps, int tree) {
+    k_level_solve_batch(const __grid_constant__ SolveBatch P, int sweeps, int tree) {
   __shared__ long long s_end[BMAX];
   __shared__ int s_lev[BMAX];
   extern __shared__ __align__(16) uint32_t s_cache[];
@@ -1003,16 +988,18 @@ __global__ void __launch_bounds__(256, NB ? MB : DCG_SOLVE_MINB)
     long long acc = 0;
     for (int m = 0; m < P.n; m++) {
       const Dev &D = P.d[m];
-      // rounds aligned at every member's finest level (round r: level maxtop - r)
-      // or, with tree & 2, at its coarsest (round r: level levels - 1 - r)
-      const int lev = (tree & 2) ? D.g.levels - 1 - round : P.maxtop - round;
-      if (lev >= 0 && lev < D.g.levels) acc += __ldcg(D.load + lev) * 64;
+      const int lev = P.lev[m];
+      if (lev >= 0) {
+        const long long load = __ldcg(D.load + lev);
+        if (load > P.cl_max[m]) acc += load * 64;
+      }
       s_lev[m] = lev;
       s_end[m] = acc;
     }
   }
   __syncthreads();
   const long long total = s_end[P.n - 1];
+  if (total == 0) return;  // the cluster solve took every level: the same in every CTA
   const unsigned nctas = gridDim.x;
   const long long stride = (long long)nctas * 256;
   const long long first = (long long)blockIdx.x * 256 + t;
@@ -1944,8 +1931,7 @@ int batch_solve_grid(int sms, int cache, int ctas_per_sm) {
   const int k = (ctas_per_sm > 0 && ctas_per_sm < occ) ? ctas_per_sm : occ;
   return k * sms;
 }
-void launch_level_solve_batch(const SolveBatch &P, int round, int sweeps, int grid, int cache, int tree,
-                              cudaStream_t st) {
+void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cache, int tree, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(256);
@@ -1958,19 +1944,19 @@ void launch_level_solve_batch(const SolveBatch &P, int round, int sweeps, int gr
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   switch (cache) {
-    case 8: cudaLaunchKernelEx(&cfg, k_level_solve_batch<8, 0>, P, round, sweeps, tree); break;
-    case 4: cudaLaunchKernelEx(&cfg, k_level_solve_batch<4, 0>, P, round, sweeps, tree); break;
-    case 3: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 0>, P, round, sweeps, tree); break;
-    case 16: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 2>, P, round, sweeps, tree); break;
-    case 32: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 3>, P, round, sweeps, tree); break;
-    case 18: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 2>, P, round, sweeps, tree); break;
-    case 19: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 2>, P, round, sweeps, tree); break;
-    case 34: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 3>, P, round, sweeps, tree); break;
-    case 35: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 3>, P, round, sweeps, tree); break;
-    case 64: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 2, 5>, P, round, sweeps, tree); break;
-    case 66: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 2, 5>, P, round, sweeps, tree); break;
-    case 83: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 2, 4, 1>, P, round, sweeps, tree); break;
-    default: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 0>, P, round, sweeps, tree); break;
+    case 8: cudaLaunchKernelEx(&cfg, k_level_solve_batch<8, 0>, P, sweeps, tree); break;
+    case 4: cudaLaunchKernelEx(&cfg, k_level_solve_batch<4, 0>, P, sweeps, tree); break;
+    case 3: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 0>, P, sweeps, tree); break;
+    case 16: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 2>, P, sweeps, tree); break;
+    case 32: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 3>, P, sweeps, tree); break;
+    case 18: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 2>, P, sweeps, tree); break;
+    case 19: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 2>, P, sweeps, tree); break;
+    case 34: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 3>, P, sweeps, tree); break;
+    case 35: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 3>, P, sweeps, tree); break;
+    case 64: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 2, 5>, P, sweeps, tree); break;
+    case 66: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 2, 5>, P, sweeps, tree); break;
+    case 83: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 2, 4, 1>, P, sweeps, tree); break;
+    default: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 0>, P, sweeps, tree); break;
   }
 }
 
