@@ -150,6 +150,17 @@ def _buf(obj, count, dtype, what, writable=False, device=False):
     raise DcgError(capi.DCG_E_INVALID, f"{what}: expected a contiguous {dt.name} {where} of {count} elements, got {got}")
 
 
+def _produced(obj, sim):
+    """Waits for torch's current stream when `obj` is a CUDA tensor and that
+    stream is not the handle's: the library reads the tensor on the handle's
+    stream, which is not ordered behind the one that computes it."""
+    if getattr(obj, "is_cuda", False):
+        import torch
+        stream = torch.cuda.current_stream(obj.device)
+        if stream.cuda_stream != getattr(sim, "_stream_ptr", None):
+            stream.synchronize()
+
+
 class Simulation:
     """One simulation handle (adaptive or uniform)."""
 
@@ -203,6 +214,7 @@ class Simulation:
 
     def set_stream(self, stream_ptr):
         self._chk(self.L.dcg_set_stream(self.h, C.c_void_p(stream_ptr)), "set_stream")
+        self._stream_ptr = stream_ptr
 
     def set_graphs(self, on):
         self._chk(self.L.dcg_set_graphs(self.h, 1 if on else 0), "set_graphs")
@@ -254,6 +266,7 @@ class Simulation:
             raise DcgError(capi.DCG_E_INVALID, f"set_heightmap: expected (nz, nx) heights, got shape {tuple(a.shape)}")
         nz, nx = int(a.shape[0]), int(a.shape[1])
         ptr, where = _buf(a, nx * nz, np.float32, "set_heightmap")
+        _produced(a, self)
         self._chk(self.L.dcg_set_heightmap(self.h, ptr, nx, nz, where), "set_heightmap")
 
     def add_velocity_noise(self, seed, amplitude):
@@ -277,6 +290,7 @@ class Simulation:
         fid = _field_id(field)
         a = values if hasattr(values, "data_ptr") else np.ascontiguousarray(values, np.float32)
         ptr, where = _buf(a, self.num_cells, np.float32, "set_field")
+        _produced(a, self)
         self._chk(self.L.dcg_set_field(self.h, fid, ptr, where), "set_field")
 
     def get_dense(self, field):
@@ -382,6 +396,7 @@ class Simulation:
     def load_state(self, buf):
         a = buf if hasattr(buf, "data_ptr") else np.ascontiguousarray(buf, np.uint8)
         ptr, where = _buf(a, self.state_bytes(), np.uint8, "load_state")
+        _produced(a, self)
         self._chk(self.L.dcg_load_state(self.h, ptr, where), "load_state")
 
     def save(self, path):
