@@ -400,7 +400,7 @@ int dcg_set_topology(dcg_sim *s, const int32_t *pos, const uint32_t *parent, con
   cudaMemsetAsync(s->D.flags, 0, B, s->stream);
   cudaMemsetAsync(s->D.nbr, 0xff, (size_t)27 * B * 4, s->stream);
   launch_build_nbr(s->D, false, s->stream);
-  return s->sync("set_topology");
+  return s->check_raster();
 }
 int dcg_get_apron(dcg_sim *s, int64_t *dst) {
   if (bad(s) || !dst || s->mode != DCG_MODE_ADAPTIVE) return DCG_E_INVALID;
@@ -778,7 +778,7 @@ int dcg_load_state(dcg_sim *s, const void *src, int32_t where) {
   }
   cudaMemsetAsync(s->D.ctr, 0, sizeof(long long) * C_COUNT, s->stream);
   cudaMemsetAsync(s->D.err, 0, 4, s->stream);
-  return s->sync("load_state");
+  return s->check_raster();
 }
 
 // ---- adjoint of the density path ------------------------------------------

@@ -39,6 +39,7 @@ struct dcg_batch {
   uint32_t *binfo = nullptr;  // block descriptions of a cascade round, BI_WORDS words per block
   uint32_t *bar = nullptr, *errw = nullptr;
   int cl_size = 0;  // cluster size of the small levels' solve (0: none)
+  std::vector<char> raster_seen;  // the members' raster flags of the captured graphs
   std::vector<unsigned long long> arena_off;
   unsigned long long arena_cells = 0;
   float *emis_arena = nullptr;  // members' emission maps, consecutive in member order
@@ -200,7 +201,9 @@ struct dcg_batch {
   }
   template <class Schedule> void solve(Schedule schedule) {
     std::vector<Dev> d(n());
+    std::vector<char> raster(n());
     for (int i = 0; i < n(); i++) {
+      raster[i] = m[i]->raster;
       d[i] = m[i]->D;
       if (planes) {  // the prolongation and the cached alpha * div read these through the descriptor
         d[i].p = d[i].e;
@@ -213,7 +216,7 @@ struct dcg_batch {
     c.sms = sms;
     c.sweeps = iters;
     c.st = stream;
-    c.run(d.data(), n(), [&](const std::vector<int> &mem, const std::vector<int> &lev, long long limit, int round) {
+    c.run(d.data(), raster.data(), n(), [&](const std::vector<int> &mem, const std::vector<int> &lev, long long limit, int round) {
       int grid = 0, cache = 0, tree = 0;
       schedule(round, grid, cache, tree);
       for (size_t g = 0; g < mem.size(); g += BMAX) {
@@ -328,6 +331,10 @@ struct dcg_batch {
   }
 
   int step(int count) {
+    std::vector<char> now;  // a member's topology from outside may change the solvers of its levels
+    for (dcg_sim *s : m) now.push_back(s->raster);
+    if (now != raster_seen) drop_graphs();
+    raster_seen = now;
     for (int i = 0; i < count; i++) {
       const int key = m[0]->vpar * 2 + m[0]->qpar;
       auto it = graphs.find(key);

@@ -257,46 +257,51 @@ __device__ inline uint32_t descend(const Dev &D, uint32_t b, int &l, int qx, int
 
 // x / 6, correctly rounded, by the method for divisors known in advance of
 // Brisebarre, Muller and Raina (IEEE Trans. Computers 53(8), 2004): q =
-// RN(x z) with z = RN(1/6), the remainder x - 6q exactly by one FMA, then
-// RN(q + r z). A zero remainder means that q is exact, which keeps the sign
-// of a zero x (most cells far from a source are zero); infinite x gives a
-// NaN remainder, and q is the quotient then too. The method assumes no
-// underflow: nonzero inputs below 2^-120 in magnitude (subnormal quotients)
-// take the IEEE division. The library's self-check (dcg_check_div6) compares
-// the result with the IEEE division over every binary32 input.
+// RN(x z) with z = RN(1/6), the negated remainder r = 6q - x exactly by one
+// FMA, then RN(q - r z). With this sign of the remainder a zero x keeps its
+// sign (r = +0, and -0 z added to q = -0 stays -0; most cells far from a
+// source are zero). The method assumes no underflow, and infinite x gives a
+// NaN remainder: nonzero inputs below 2^-120 in magnitude (subnormal
+// quotients) and infinities take the IEEE division. The library's self-check
+// (dcg_check_div6) compares the result with the IEEE division over every
+// binary32 input.
+__device__ __forceinline__ bool div6_rare(float x) {
+  const float a = fabsf(x);
+  return (a < 0x1p-120f && x != 0.f) || a == __int_as_float(0x7f800000);
+}
 __device__ __forceinline__ float div6(float x) {
   const float z = 0x1.555556p-3f;
   const float q = __fmul_rn(x, z);
-  const float r = fmaf(-q, 6.f, x);
-  const float y = fmaf(r, z, q);
-  float o = fabsf(r) > 0.f ? y : q;
-  if (fabsf(x) < 0x1p-120f && x != 0.f) o = x / 6.f;
+  const float r = fmaf(q, 6.f, -x);
+  float o = fmaf(-r, z, q);
+  if (div6_rare(x)) o = x / 6.f;
   return o;
 }
 
 // div6 of the components of N pairs with packed FP32x2 operations (each
 // component the correctly rounded operation of div6's scalar form, so the
-// results are div6's). One test of the smallest magnitude sends the lane to
-// the component-wise subnormal test, which developed flows rarely need.
+// results are div6's). The smallest and largest magnitudes send the lane to
+// the component-wise test, which developed flows rarely need.
 __device__ __noinline__ inline float div6_small(float x) { return x / 6.f; }
 template <int N> __device__ __forceinline__ void div6_pairs(float2 (&x)[N]) {
-  const float2 z = make_float2(0x1.555556p-3f, 0x1.555556p-3f);
+  const float2 z = make_float2(0x1.555556p-3f, 0x1.555556p-3f), nz = make_float2(-0x1.555556p-3f, -0x1.555556p-3f);
   float2 o[N];
-  float small = fminf(fabsf(x[0].x), fabsf(x[0].y));
+  float small = fminf(fabsf(x[0].x), fabsf(x[0].y)), large = fmaxf(fabsf(x[0].x), fabsf(x[0].y));
 #pragma unroll
   for (int i = 0; i < N; i++) {
     const float2 q = __fmul2_rn(x[i], z);
-    const float2 r = __ffma2_rn(q, make_float2(-6.f, -6.f), x[i]);  // x - 6 q, exactly as fmaf(-q, 6, x)
-    const float2 y = __ffma2_rn(r, z, q);
-    o[i].x = fabsf(r.x) > 0.f ? y.x : q.x;
-    o[i].y = fabsf(r.y) > 0.f ? y.y : q.y;
-    if (i > 0) small = fminf(small, fminf(fabsf(x[i].x), fabsf(x[i].y)));
+    const float2 r = __ffma2_rn(q, make_float2(6.f, 6.f), make_float2(-x[i].x, -x[i].y));  // 6 q - x, exactly
+    o[i] = __ffma2_rn(r, nz, q);
+    if (i > 0) {
+      small = fminf(fminf(small, fabsf(x[i].x)), fabsf(x[i].y));
+      large = fmaxf(fmaxf(large, fabsf(x[i].x)), fabsf(x[i].y));
+    }
   }
-  if (small < 0x1p-120f) {
+  if (small < 0x1p-120f || large > 0x1.fffffep127f) {
 #pragma unroll
     for (int i = 0; i < N; i++) {
-      if (fabsf(x[i].x) < 0x1p-120f && x[i].x != 0.f) o[i].x = div6_small(x[i].x);
-      if (fabsf(x[i].y) < 0x1p-120f && x[i].y != 0.f) o[i].y = div6_small(x[i].y);
+      if (div6_rare(x[i].x)) o[i].x = div6_small(x[i].x);
+      if (div6_rare(x[i].y)) o[i].y = div6_small(x[i].y);
     }
   }
 #pragma unroll
@@ -307,7 +312,6 @@ __device__ __forceinline__ float2 div6x2(float2 x) {
   div6_pairs(v);
   return v[0];
 }
-__device__ __forceinline__ void div6x8(float2 (&x)[4]) { div6_pairs(x); }
 
 __device__ inline int dir_of(int a) { return a == 0 ? 0 : (a == AW - 1 ? 2 : 1); }
 

@@ -127,22 +127,63 @@ int cluster_solve_size();
 long long cluster_solve_blocks(int csize);
 void launch_cluster_solve(ClusterSolve &P, int max_csize, long long max_blocks, int sms, cudaStream_t st);
 
+// k_dense.cu: sweeps of dense boxes of A (contiguous) x B x M cells, several
+// per pass over memory
+struct DenseLevel {
+  const float *in, *rhs;
+  float *out, *out2;  // the result; the iterate before the last (last pass), or null
+  int A, B, M;
+  int nq, nr, ta, tb, clen;  // tile: quads along A, row pairs along B; tiles; planes per chunk
+  int zero, blocks;          // the input is zero; the outputs take the block layout (ra, rb blocks along A, B)
+  int ra, rb;
+  float nalpha;
+};
+struct DensePass {
+  int n;
+  int end[BMAX];  // cumulative CTAs
+  DenseLevel l[BMAX];
+};
+struct DenseCopyLevel {
+  int X, Y, Z;
+  const float *p, *coarse, *div;  // block layouts; coarse: the parent level's p, or null (no prolongation)
+  float *lin, *rhs;
+  float alpha;
+};
+struct DenseCopy {
+  int n;
+  int end[BMAX];
+  DenseCopyLevel l[BMAX];
+};
+struct DenseSweep {
+  int A, B, M;
+  const float *src, *rhs;
+  float *x0, *x1, *dst, *dst2;
+  float nalpha;
+  bool zero, blocks;
+};
+void launch_dense_sweeps(const DenseSweep *v, int n, int sweeps, bool uniform, int sms, cudaStream_t st);
+void launch_dense_solve(const Dev *d, const int *lev, int n, int prolong, int sweeps, int sms, cudaStream_t st);
+
 // Host schedule of a cascade over any number of simulations: every level of
 // every member, coarse to fine, each by the solver that suits it. The levels
 // whose budget a cluster holds go to the cluster solve, runs of them in one
-// launch; a larger level goes there too while its allocated blocks fit
-// (known on the device only), else to `general`, which is launched behind it
-// and leaves what the cluster solve took.
+// launch; larger levels that are allocated in full, in raster order, to the
+// dense solve; a larger sparse level goes to the cluster solve too while its
+// allocated blocks fit (known on the device only), else to `general`, which is
+// launched behind it and leaves what the cluster solve took.
 struct Cascade {
   int csize = 0;  // cluster size of the device (0: no cluster solve)
   int sms = 148;
   int sweeps = 0, prolong = 1;
   cudaStream_t st = nullptr;
+  // blocks that make the dense solve the faster one (a box of 8192 blocks: 6.9
+  // us per sweep, grid-wide 5.3; of 32768: 8.3 and 9.3)
+  static constexpr long long kDenseBlocks = 16384;
   long long limit() const { return csize > 0 ? cluster_solve_blocks(csize) : 0; }
   // general(members, levels, limit, round): solve levels[i] of members[i]
   // unless at most `limit` of its blocks are allocated
-  // only >= 0: that level alone
-  template <class General> void run(const Dev *d, int n, General general, int only = -1) const;
+  // raster[i]: member i's full levels lie in raster order; only >= 0: that level alone
+  template <class General> void run(const Dev *d, const char *raster, int n, General general, int only = -1) const;
 };
 
 // self-check of the solver's division by six: bad[0] += mismatches, bad[1] = min mismatching input
@@ -153,6 +194,9 @@ int launch_barrier_probe(uint32_t *bar, uint32_t *errw, unsigned limit, unsigned
 void launch_init_blocks(const Dev &D, cudaStream_t st);
 void launch_activate_level(const Dev &D, int level, cudaStream_t st);
 void launch_build_nbr(const Dev &D, bool only_if_touched, cudaStream_t st);
+// *bad = 1 unless every level whose budget covers its block grid is allocated
+// in full, in raster order, with parents and face neighbours to match
+void launch_check_raster(const Dev &D, uint32_t *bad, cudaStream_t st);
 void launch_adapt(const Dev &D, const SortScratch &s, uint32_t *keys, uint32_t *vals,
                   uint32_t *keys2, uint32_t *vals2, int sms, cudaStream_t st);
 // launch_adapt for up to BMAX members, one launch per adaptation kernel;
@@ -208,7 +252,7 @@ void launch_u_fluidity(const UDev &U, cudaStream_t st);
 void launch_u_sources(const UDev &U, cudaStream_t st);
 void launch_u_advect_velocity(const UDev &U, cudaStream_t st);
 void launch_u_advect_scalars(const UDev &U, cudaStream_t st);
-void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, cudaStream_t st);
+void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, int sms, cudaStream_t st);
 void launch_u_add_noise(const UDev &U, unsigned long long seed, float amp, cudaStream_t st);
 void launch_u_stats(const UDev &U, cudaStream_t st);
 void launch_render_adaptive(const Dev &D, const RenderP &R, float4 *out, cudaStream_t st);

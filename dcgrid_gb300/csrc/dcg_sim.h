@@ -26,38 +26,50 @@ int idiv_up(int a, int b) { return (a % b != 0) ? (a / b + 1) : (a / b); }
 }  // namespace
 
 namespace dcg {
-template <class General> void Cascade::run(const Dev *d, int n, General general, int only) const {
-  // The grid-wide solve shares its barriers over the members of a round, the
-  // clusters share nothing: a batch with more blocks than clusters hold at once
-  // stays with it (16 plumes of 64^3 to 256^3: 9.9 ms per step, 11.6 ms with
-  // clusters; 10 plumes of 32^3 to 64^3: 0.54 ms, 0.41 ms with clusters).
-  long long lim = limit(), all = 0;
-  for (int i = 0; i < n; i++)
-    for (int l = 0; l < d[i].g.levels; l++) all += d[i].g.budget[l];
-  if (n > 1 && all > 8 * lim) lim = 0;
+template <class General>
+void Cascade::run(const Dev *d, const char *raster, int n, General general, int only) const {
+  const long long lim = limit();
   std::vector<int> cur(n);
   for (int i = 0; i < n; i++) cur[i] = only >= 0 ? only : d[i].g.levels - 1;
   const int last = only >= 0 ? only : 0;
-  for (int round = 0;; round++) {
-    std::vector<int> mem, hi, lo, gm, gl;  // cluster runs; members and levels left to `general`
+  auto full = [&](int i) { return d[i].g.budget[cur[i]] == d[i].g.full[cur[i]]; };
+  for (int round = 0; std::any_of(cur.begin(), cur.end(), [&](int l) { return l >= last; });) {
+    // full levels first, while together they have work for the dense solve
+    std::vector<Dev> dd;
+    std::vector<int> dl, dm;
     long long blocks = 0;
-    bool left = false;
+    for (int i = 0; i < n; i++)
+      if (cur[i] >= last && raster[i] && sweeps > 0 && full(i)) {
+        dd.push_back(d[i]);
+        dl.push_back(cur[i]);
+        dm.push_back(i);
+        blocks += d[i].g.budget[cur[i]];
+      }
+    if (blocks >= kDenseBlocks) {
+      launch_dense_solve(dd.data(), dl.data(), (int)dd.size(), prolong, sweeps, sms, st);
+      for (int i : dm) cur[i]--;
+      continue;
+    }
+    // then runs of levels that a cluster holds, and behind them one larger level each
+    std::vector<int> mem, hi, lo, gm, gl;
+    blocks = 0;
     for (int i = 0; i < n; i++) {
       if (cur[i] < last) continue;
-      left = true;
       const Geom &g = d[i].g;
       const int top = cur[i];
       int l = top;
       while (l >= last && g.budget[l] <= lim) blocks = std::max(blocks, g.budget[l--]);
-      if (l >= last) {
-        if (lim > 0 && g.budget[l] < g.full[l]) blocks = lim;
+      cur[i] = l;
+      if (l < last) {
+        l = last;
+      } else if (full(i) && raster[i] && g.budget[l] >= kDenseBlocks && sweeps > 0) {
+        l++;  // the dense solve's, next
+      } else {
         gm.push_back(i);
         gl.push_back(l);
         cur[i] = l - 1;
-        if (!(lim > 0 && g.budget[l] < g.full[l])) l++;  // allocated in full: never fits
-      } else {
-        cur[i] = -1;
-        l = last;
+        if (lim > 0 && g.budget[l] < g.full[l]) blocks = lim;
+        else l++;  // allocated in full: never fits a cluster
       }
       if (l <= top) {
         mem.push_back(i);
@@ -65,7 +77,6 @@ template <class General> void Cascade::run(const Dev *d, int n, General general,
         lo.push_back(l);
       }
     }
-    if (!left) return;
     for (size_t g = 0; g < mem.size(); g += BMAX) {
       ClusterSolve P{};
       P.n = (int)std::min<size_t>(BMAX, mem.size() - g);
@@ -79,7 +90,7 @@ template <class General> void Cascade::run(const Dev *d, int n, General general,
       }
       launch_cluster_solve(P, csize, blocks, sms, st);
     }
-    if (!gm.empty()) general(gm, gl, lim, round);
+    if (!gm.empty()) general(gm, gl, lim, round++);
   }
 }
 }  // namespace dcg
@@ -134,6 +145,9 @@ struct dcg_sim {
   int ls_epoch = 3;
   int ls_grid_staged = 0;  // CTAs of the staged solve
   int cl_size = 0;         // cluster size of the small levels' solve (0: none)
+  // the full levels lie in raster order, as created (a caller's topology or
+  // state may say otherwise: check_raster)
+  char raster = 1;
   // level solve of single simulations: pipelined staged sweeps, two tile buffers,
   // block descriptions cached in 3 x 8 KB of shared memory when they fit.
   // Variant 19 (3 CTAs per SM, two blocks per claim); variant 83 (4 CTAs per
@@ -412,9 +426,29 @@ struct dcg_sim {
     return DCG_OK;
   }
 
+  void drop_graphs() {
+    for (auto &kv : graphs) cudaGraphExecDestroy(kv.second);
+    graphs.clear();
+  }
+  void set_raster(char now) {
+    if (now != raster) drop_graphs();  // they hold the solvers chosen for the old order
+    raster = now;
+  }
+  // after a topology from outside: whether the dense solve applies
+  int check_raster() {
+    uint32_t bad = 1;
+    int rc;
+    launch_check_raster(D, D.err + 1, stream);
+    if ((rc = cuda(cudaMemcpyAsync(&bad, D.err + 1, 4, cudaMemcpyDeviceToHost, stream), "raster check"))) return rc;
+    if ((rc = sync("raster check"))) return rc;
+    set_raster(bad ? 0 : 1);
+    return DCG_OK;
+  }
+
   // FluidSimulationDCGrid::reset + init (fluid_simulation_dcgrid.cu:190-261)
   int reset_adaptive() {
     int rc;
+    set_raster(1);
     vpar = qpar = 0;
     bind_parity();
     const size_t nc = (size_t)D.g.B * BV;
@@ -586,7 +620,7 @@ struct dcg_sim {
     c.sweeps = sweeps;
     c.prolong = prolong;
     c.st = stream;
-    c.run(&d, 1, [&](const std::vector<int> &, const std::vector<int> &lev, long long limit, int) {
+    c.run(&d, &raster, 1, [&](const std::vector<int> &, const std::vector<int> &lev, long long limit, int) {
       solve_staged(d, lev[0], prolong, sweeps, limit);
     });
   }
@@ -598,7 +632,7 @@ struct dcg_sim {
     c.sweeps = sweeps;
     c.prolong = 0;
     c.st = stream;
-    c.run(&D, 1, [&](const std::vector<int> &, const std::vector<int> &lev, long long limit, int) {
+    c.run(&D, &raster, 1, [&](const std::vector<int> &, const std::vector<int> &lev, long long limit, int) {
       solve_staged(D, lev[0], 0, sweeps, limit);
     }, level);
   }
@@ -723,7 +757,7 @@ struct dcg_sim {
   void u_project(bool local) {
     const int top_pairs = P.ref_compat ? 2 : P.jacobi_iters / 2;
     const int pairs = local ? (P.ref_compat ? 5 : P.jacobi_iters / 2) : (P.ref_compat ? 1 : P.jacobi_iters / 2);
-    launch_u_project(U, top_pairs, pairs, local, stream);
+    launch_u_project(U, top_pairs, pairs, local, sms, stream);
   }
   void u_advect_scalars() {
     launch_u_advect_scalars(U, stream);

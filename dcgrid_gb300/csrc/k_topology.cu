@@ -653,6 +653,32 @@ void launch_activate_level(const Dev &D, int level, cudaStream_t st) {
   const long long nb = (long long)D.g.rx[level] * D.g.ry[level] * D.g.rz[level];
   k_activate_level<<<grid_for(nb * 64), 256, 0, st>>>(D, level);
 }
+__global__ void __launch_bounds__(256) k_check_raster(Dev D, int level, uint32_t *bad) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t == 0 && D.load[level] != D.g.full[level]) *bad = 1u;
+  if (t >= D.g.full[level]) return;
+  const int ry = D.g.ry[level], rz = D.g.rz[level];
+  const int x = BW * (int)(t / ((long long)ry * rz)), y = BW * (int)((t / rz) % ry), z = BW * (int)(t % rz);
+  const long long b = D.g.off[level] + t;
+  const int4 p = D.pos[b];
+  bool ok = p.x == x && p.y == y && p.z == z && p.w == level;
+  if (level < D.g.levels - 1)
+    ok = ok && D.parent[b] == 8u * dense_index(D.g, x / 2, y / 2, z / 2, level + 1) +
+                                  (uint32_t)((x % (2 * BW)) + (y % (2 * BW)) / 2 + (z % (2 * BW)) / 4);
+  const int sc = 1 << level;
+  for (int d = 0; d < 27; d++) {
+    const int dx = d / 9 - 1, dy = (d / 3) % 3 - 1, dz = d % 3 - 1;
+    const int qx = x + BW * dx, qy = y + BW * dy, qz = z + BW * dz;
+    const bool out = qx < 0 || qy < 0 || qz < 0 || qx * sc >= D.g.gx || qy * sc >= D.g.gy || qz * sc >= D.g.gz;
+    if (d != 13) ok = ok && D.nbr[27 * b + d] == (out ? OUT : dense_index(D.g, qx, qy, qz, level));
+  }
+  if (!ok) *bad = 1u;
+}
+void launch_check_raster(const Dev &D, uint32_t *bad, cudaStream_t st) {
+  cudaMemsetAsync(bad, 0, sizeof(uint32_t), st);
+  for (int l = D.g.sparse; l < D.g.levels; l++)
+    k_check_raster<<<(unsigned)((D.g.full[l] + 255) / 256), 256, 0, st>>>(D, l, bad);
+}
 void launch_build_nbr(const Dev &D, bool only_if_touched, cudaStream_t st) {
   k_build_nbr<<<grid_for(D.g.B * 27), 256, 0, st>>>(D, only_if_touched ? 1 : 0);
 }

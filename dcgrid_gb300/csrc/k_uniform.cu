@@ -185,14 +185,11 @@ __global__ void __launch_bounds__(256) k_u_jacobi(UDev U, int level, const float
   dst[idx] = div6(src[il] + src[ir] + src[id] + src[iu] + src[ib] + src[iff] - alpha * U.div[idx]);
 }
 
-// k_uniform_prolongate (uniformgrid_fluid.cu:206-237)
-__global__ void __launch_bounds__(256) k_u_prolongate(UDev U, int level) {
+// k_uniform_prolongate (uniformgrid_fluid.cu:206-237): one cell, index i of its level
+__device__ inline float u_prolong(const UDev &U, int level, long long i) {
   const int s = 1 << level;
   const int w = U.gx / s, h = U.gy / s, d = U.gz / s;
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (long long)w * h * d) return;
   const int x = (int)(i % w), y = (int)((i / w) % h), z = (int)(i / ((long long)w * h));
-  const size_t idx = (size_t)U.mip_off[level] + (size_t)i;
   const size_t i000 = umip(U, x / 2, y / 2, z / 2, level + 1);
   const int sx = (x == 0 || x == w - 1) ? 0 : 2 * (x % 2) - 1;
   const int sy = (y == 0 || y == h - 1) ? 0 : 2 * (y % 2) - 1;
@@ -205,8 +202,59 @@ __global__ void __launch_bounds__(256) k_u_prolongate(UDev U, int level) {
   const size_t i110 = i100 + (long long)sy * (w / 2);
   const size_t i111 = i110 + sx;
   const float *P = U.p;
-  U.p[idx] = (27.f * P[i000] + 9.f * (P[i001] + P[i010] + P[i100]) + 3.f * (P[i011] + P[i101] + P[i110]) +
-              P[i111]) / 64.f;
+  return (27.f * P[i000] + 9.f * (P[i001] + P[i010] + P[i100]) + 3.f * (P[i011] + P[i101] + P[i110]) + P[i111]) / 64.f;
+}
+__global__ void __launch_bounds__(256) k_u_prolongate(UDev U, int level, float *out) {
+  const int s = 1 << level;
+  const long long n = (long long)(U.gx / s) * (U.gy / s) * (U.gz / s);
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = u_prolong(U, level, i);
+}
+
+// Small mip levels hi..lo (coarse to fine, each of at most SB_CELLS cells) by
+// one CTA, a level's prolongation and all its sweeps in shared memory: two
+// planes and a byte per cell that says on which faces of the box it lies. One
+// launch and a CTA barrier per sweep instead of a launch per sweep (4.1 us):
+// a level of 24^3 cells takes about 1.5 us per sweep, 12^3 and below 0.4 us.
+// Bound by the shared-memory reads of one SM.
+constexpr int SB_THREADS = 1024, SB_CELLS = 24 * SB_THREADS;
+constexpr int SB_SMEM = SB_CELLS * 9;
+__global__ void __launch_bounds__(SB_THREADS, 1) k_u_small(UDev U, int hi, int lo, int sweeps_hi, int sweeps) {
+  extern __shared__ __align__(16) float sb[];
+  unsigned char *face = reinterpret_cast<unsigned char *>(sb + 2 * SB_CELLS);
+  for (int level = hi; level >= lo; level--) {
+    const int s = 1 << level;
+    const int w = U.gx / s, h = U.gy / s, d = U.gz / s, wh = w * h, n = wh * d;
+    const size_t off = (size_t)U.mip_off[level];
+    const float alpha = U.ph.dx * U.ph.dx * (float)s * (float)s;
+    const bool top = level == U.levels - 1;
+    const int todo = level == hi ? sweeps_hi : sweeps;
+    for (int i = threadIdx.x; i < n; i += SB_THREADS) {
+      const int x = i % w, y = (i / w) % h, z = i / wh;
+      face[i] = (unsigned char)((x == 0) | (x == w - 1) << 1 | (y == 0) << 2 | (y == h - 1) << 3 | (z == 0) << 4 |
+                                (z == d - 1) << 5);
+      sb[i] = top ? 0.f : u_prolong(U, level, i);
+      sb[SB_CELLS + i] = 0.f;
+    }
+    for (int it = 0; it < todo; it++) {
+      const float *src = sb + (it & 1) * SB_CELLS;
+      float *dst = sb + ((it & 1) ^ 1) * SB_CELLS;
+      __syncthreads();
+      for (int i = threadIdx.x; i < n; i += SB_THREADS) {
+        const unsigned f = face[i];
+        const float *c = src + i;
+        const float l = c[(f & 1u) ? 0 : -1], r = c[(f & 2u) ? 0 : 1], dn = c[(f & 4u) ? 0 : -w],
+                    up = c[(f & 8u) ? 0 : w], bk = c[(f & 16u) ? 0 : -wh], fw = c[(f & 32u) ? 0 : wh];
+        dst[i] = div6(l + r + dn + up + bk + fw - alpha * U.div[off + i]);
+      }
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < n; i += SB_THREADS) {
+      U.p[off + i] = sb[i];  // an even number of sweeps
+      if (todo > 0) U.pt[off + i] = sb[SB_CELLS + i];
+    }
+    __syncthreads();  // the next level's prolongation reads p
+  }
 }
 
 // k_uniform_apply_pressure (uniformgrid_fluid.cu:239-260)
@@ -258,28 +306,47 @@ void launch_u_advect_velocity(const UDev &U, cudaStream_t st) {
 void launch_u_advect_scalars(const UDev &U, cudaStream_t st) {
   k_u_advect_scalars<<<ugrid(U.nc), 256, 0, st>>>(U);
 }
+// The sweeps of one mip level from its prolongation (or from zero) into p, the
+// iterate before the last into p~. Larger levels take the dense passes from
+// U.tv[0], where their prolongation goes, with U.tv[0] and U.tv[1], free until
+// the next velocity advection, as scratch; below kDenseCells a launch per
+// sweep is faster (48^3: 4.1 against 4.7 us per sweep; 64^3: 6.1 and 5.6; 192^3:
+// 55 and 13).
+constexpr long long kDenseCells = 200000;
+static void u_sweeps(const UDev &U, int level, int sweeps, bool zero, int sms, cudaStream_t st) {
+  const long long n = ucells(U, level);
+  const size_t o = (size_t)U.mip_off[level];
+  const bool dense = n > kDenseCells && sweeps > 0;
+  if (!zero) k_u_prolongate<<<ugrid(n), 256, 0, st>>>(U, level, dense ? U.tv[0] : U.p + o);
+  if (dense) {
+    const int s = 1 << level;
+    const float alpha = U.ph.dx * U.ph.dx * (float)s * (float)s;
+    const DenseSweep v{U.gx / s,  U.gy / s,  U.gz / s,  U.tv[0], U.div + o, U.tv[0],
+                       U.tv[1],   U.p + o,   U.pt + o,  -alpha,  zero,      false};
+    launch_dense_sweeps(&v, 1, sweeps, true, sms, st);
+    return;
+  }
+  for (int i = 0; i < sweeps / 2; i++) {
+    k_u_jacobi<<<ugrid(n), 256, 0, st>>>(U, level, U.p, U.pt);
+    k_u_jacobi<<<ugrid(n), 256, 0, st>>>(U, level, U.pt, U.p);
+  }
+}
 // FluidSimulationUniform::project / projectLocal (fluid_simulation_uniform.cu:96-135)
-void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, cudaStream_t st) {
+void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, int sms, cudaStream_t st) {
   k_u_divergence<<<ugrid(U.nc), 256, 0, st>>>(U);
   if (local) {
-    for (int i = 0; i < pairs; i++) {
-      k_u_jacobi<<<ugrid(U.nc), 256, 0, st>>>(U, 0, U.p, U.pt);
-      k_u_jacobi<<<ugrid(U.nc), 256, 0, st>>>(U, 0, U.pt, U.p);
-    }
+    u_sweeps(U, 0, 2 * pairs, true, sms, st);
   } else {
     for (int l = 1; l < U.levels; l++) k_u_restrict<<<ugrid(ucells(U, l)), 256, 0, st>>>(U, l);
     const int top = U.levels - 1;
-    for (int i = 0; i < top_pairs; i++) {
-      k_u_jacobi<<<ugrid(ucells(U, top)), 256, 0, st>>>(U, top, U.p, U.pt);
-      k_u_jacobi<<<ugrid(ucells(U, top)), 256, 0, st>>>(U, top, U.pt, U.p);
+    int l = top;
+    while (l >= 0 && ucells(U, l) <= SB_CELLS) l--;
+    if (l < top) {  // the levels that one CTA holds
+      static const cudaError_t ok = cudaFuncSetAttribute(k_u_small, cudaFuncAttributeMaxDynamicSharedMemorySize, SB_SMEM);
+      if (ok == cudaSuccess) k_u_small<<<1, SB_THREADS, SB_SMEM, st>>>(U, top, l + 1, 2 * top_pairs, 2 * pairs);
+      else l = top;
     }
-    for (int l = U.levels - 2; l >= 0; l--) {
-      k_u_prolongate<<<ugrid(ucells(U, l)), 256, 0, st>>>(U, l);
-      for (int i = 0; i < pairs; i++) {
-        k_u_jacobi<<<ugrid(ucells(U, l)), 256, 0, st>>>(U, l, U.p, U.pt);
-        k_u_jacobi<<<ugrid(ucells(U, l)), 256, 0, st>>>(U, l, U.pt, U.p);
-      }
-    }
+    for (; l >= 0; l--) u_sweeps(U, l, 2 * (l == top ? top_pairs : pairs), l == top, sms, st);
   }
   k_u_apply_pressure<<<ugrid(U.nc), 256, 0, st>>>(U);
 }

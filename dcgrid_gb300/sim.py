@@ -209,6 +209,7 @@ class Simulation:
     def set_mode(self, mode):
         """The reference's adaptive/uniform switch: recreate, state dropped."""
         self._chk(self.L.dcg_set_mode(C.byref(self.h), mode), "set_mode")
+        self._stream_ptr = None
         self.mode = mode
         self._chk(self.L.dcg_get_info(self.h, C.byref(self.info)), "get_info")
 
