@@ -231,9 +231,12 @@ __global__ void __launch_bounds__(256) k_scores_fields(Dev D) { scores_fields_bo
 
 // k_dcgrid_accumulate_subblock_scores (dcgrid_adaptation.cu:42-63); with
 // ref_compat the reference's ninth summand s[8] is included.
+// (it opens the adaptation: the block flags and the counters are cleared here)
 __device__ __forceinline__ void block_scores_body(const Dev &D, unsigned bx, unsigned gx) {
   const long long b = (long long)bx * blockDim.x + threadIdx.x;
+  if (b < C_COUNT) D.ctr[b] = 0;
   if (b >= D.g.B) return;
+  D.flags[b] = 0;
   D.bs[b] = -FLT_MAX;
   const int level = D.pos[b].w;
   if (level < 0 || level_blocked(D, level)) return;
@@ -642,6 +645,391 @@ __device__ __forceinline__ void propagate_body(const Dev &D, int level, unsigned
 }
 __global__ void __launch_bounds__(256) k_propagate(Dev D, int level) { propagate_body(D, level, blockIdx.x, gridDim.x); }
 
+// ------------------------------------------------------------ decisions by one CTA
+// The moves and the refinements of one simulation of up to kDecideBlocks
+// blocks, each phase by one CTA in one launch. The decisions need the best
+// few candidates of two lists, in order; sorting both lists in full took 32
+// dependent launches per sparse level (250 us of a small scene's step and
+// more than its kernels' work). Here the CTA reads the lists once for their
+// best elements: when the first pair does not match, as in most steps, the
+// phase is over. Else it counts the elements that can match at all (a block
+// below the best destination, a destination above the worst block), selects
+// the best DC_LIST of each by radix histograms of (key, index), sorts those in
+// shared memory and walks the pairs, DC_LIST at a time. The 64-bit key
+// (score key, index) is unique, so the order is the stable sort's: equal
+// scores by ascending index.
+// What bounds it: one SM's reads of the lists (about 10 us per pass over
+// 262144 scores) and barriers. Whole adaptations, sorts -> this: 454 blocks
+// 248 -> 39 us, 9855 blocks 284 -> 37, the 40000-block cloud 700 -> 91, 16
+// plumes of up to 98304 blocks 985 -> 720 (one CTA per member). A list of half
+// a million scores would take one SM as long as the sorts take the GPU; larger
+// simulations keep the sorts.
+constexpr int DC_THREADS = 1024, DC_LIST = 4096;
+constexpr int DC_SMEM = 2 * DC_LIST * 8;
+constexpr long long kDecideBlocks = 131072;
+typedef unsigned long long u64;
+
+__device__ __forceinline__ uint32_t block_key(float s) { return s < 0.f ? 0xFFFFFFFFu : (__float_as_uint(s) & 0x7FFFFFFFu); }
+__device__ __forceinline__ uint32_t dest_key(float s) {
+  uint32_t u = s == 0.f ? 0u : __float_as_uint(s);
+  u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);  // order-preserving map
+  return ~u;                                       // descending
+}
+__device__ __forceinline__ float dest_score(uint32_t key) {
+  const uint32_t u = ~key;
+  return __uint_as_float((u & 0x80000000u) ? u & 0x7FFFFFFFu : ~u);
+}
+
+// calls f(i, scores[i]) for every i < n, several loads in flight per thread
+template <class F> __device__ __forceinline__ void dc_each(const float *scores, long long n, F f) {
+  long long i = threadIdx.x;
+  for (; i + 7 * DC_THREADS < n; i += 8 * DC_THREADS) {
+    float v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) v[k] = scores[i + k * DC_THREADS];
+#pragma unroll
+    for (int k = 0; k < 8; k++) f(i + k * DC_THREADS, v[k]);
+  }
+  for (; i < n; i += DC_THREADS) f(i, scores[i]);
+}
+__device__ __forceinline__ u64 dc_min(u64 v) {  // over the CTA
+  __shared__ u64 ws[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const u64 t = __shfl_xor_sync(0xffffffffu, v, o);
+    v = t < v ? t : v;
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = ws[threadIdx.x & 31];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const u64 t = __shfl_xor_sync(0xffffffffu, v, o);
+    v = t < v ? t : v;
+  }
+  return v;
+}
+// exclusive prefix of v over the CTA's threads, the total in *total
+__device__ __forceinline__ uint32_t dc_scan(uint32_t v, uint32_t *total) {
+  __shared__ uint32_t ws[32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();
+  if (lane == 31) ws[w] = x;
+  __syncthreads();
+  uint32_t t = ws[lane];
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
+    if (lane >= o) t += y;
+  }
+  *total = __shfl_sync(0xffffffffu, t, 31);
+  const uint32_t before = __shfl_sync(0xffffffffu, t, (w + 31) & 31);
+  return (w ? before : 0u) + x - v;
+}
+// A list of scores: item i has the 64-bit key (KEY(score) << 32 | first + i);
+// in(score) tells whether it takes part.
+template <class Key, class In> struct DcList {
+  const float *s;
+  long long n;
+  uint32_t first;
+  Key key;
+  In in;
+  __device__ __forceinline__ u64 full(long long i, float v) const { return ((u64)key(v) << 32) | (first + (uint32_t)i); }
+};
+// The largest of the `need` smallest keys above `above` (need is at least 1 and
+// at most their number): radix selection, 11 bits per pass, ending as soon as
+// a digit's bin is taken whole.
+template <class L> __device__ __forceinline__ u64 dc_select(const L &l, u64 above, bool any, uint32_t need) {
+  __shared__ uint32_t hist[2048];
+  __shared__ uint32_t s_bin, s_before, s_count;
+  u64 prefix = 0;
+  for (int shift = 53;; shift = shift > 11 ? shift - 11 : 0) {
+    const int bits = shift == 0 ? 9 : 11;  // 64 = 5 * 11 + 9
+    __syncthreads();
+    hist[threadIdx.x] = hist[threadIdx.x + 1024] = 0;
+    __syncthreads();
+    dc_each(l.s, l.n, [&](long long i, float v) {
+      if (!l.in(v)) return;
+      const u64 k = l.full(i, v);
+      if (any && k <= above) return;
+      if (shift + bits < 64 && (k >> (shift + bits)) != prefix) return;
+      atomicAdd(&hist[(uint32_t)(k >> shift) & ((1u << bits) - 1u)], 1u);
+    });
+    __syncthreads();
+    const uint32_t a = hist[2 * threadIdx.x], b = hist[2 * threadIdx.x + 1];
+    uint32_t total;
+    const uint32_t ex = dc_scan(a + b, &total);
+    if (ex < need && ex + a + b >= need) {
+      const bool second = ex + a < need;
+      s_bin = 2 * threadIdx.x + (second ? 1 : 0);
+      s_before = ex + (second ? a : 0);
+      s_count = second ? b : a;
+    }
+    __syncthreads();
+    prefix = (prefix << bits) | s_bin;
+    need -= s_before;
+    if (shift == 0) return prefix;
+    if (need == s_count) return (prefix << shift) | ((1ull << shift) - 1ull);
+  }
+}
+// ascending bitonic sort of buf[0, n) (n <= DC_LIST; padded to a power of two)
+__device__ __forceinline__ void dc_sort(u64 *buf, int n) {
+  int m = 2;
+  while (m < n) m *= 2;
+  for (int i = n + threadIdx.x; i < m; i += DC_THREADS) buf[i] = ~0ull;
+  for (int k = 2; k <= m; k *= 2)
+    for (int j = k / 2; j > 0; j /= 2) {
+      __syncthreads();
+      for (int t = threadIdx.x; t < m / 2; t += DC_THREADS) {
+        const int i = 2 * t - (t & (j - 1)), o = i + j;  // i has bit j clear
+        const u64 a = buf[i], b = buf[o];
+        if ((a > b) == ((i & k) == 0)) {
+          buf[i] = b;
+          buf[o] = a;
+        }
+      }
+    }
+  __syncthreads();
+}
+// the next `want` members (at most DC_LIST) of the `left` that the list has
+// above `above`: sorted into buf, their number returned
+template <class L> __device__ __forceinline__ int dc_take(const L &l, u64 above, bool any, long long left, long long want, u64 *buf) {
+  __shared__ uint32_t s_n;
+  const uint32_t k = (uint32_t)min(min(want, left), (long long)DC_LIST);
+  const u64 limit = left > (long long)k ? dc_select(l, above, any, k) : ~0ull;
+  __syncthreads();
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  dc_each(l.s, l.n, [&](long long i, float v) {
+    if (!l.in(v)) return;
+    const u64 key = l.full(i, v);
+    if ((any && key <= above) || key > limit) return;
+    const uint32_t at = atomicAdd(&s_n, 1u);
+    if (at < (uint32_t)DC_LIST) buf[at] = key;
+  });
+  __syncthreads();
+  const int n = (int)min(s_n, (uint32_t)DC_LIST);
+  dc_sort(buf, n);
+  return n;
+}
+
+// the moves of one level (move_setup, keys, sorts, match and commit above)
+__device__ __forceinline__ void dc_moves(const Dev &D, int L, u64 *lb, u64 *ld) {
+  __shared__ uint32_t s_cnt[2], s_fail;
+  const long long d0 = D.g.budget[L], d1 = 8 * D.g.budget[L + 1];
+  long long l = d0 < d1 ? d0 : d1;
+  l = min(l, D.load[L]);
+  l = min(l, D.g.full[L] - D.load[L]);
+  if (D.move_limit[L] > 0) l = min(l, D.move_limit[L]);
+  const long long base = D.ctr[C_MOVES];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    D.ctr[C_MOVE_LIMIT] = l;
+    D.ctr[C_MATCHES] = l;
+    D.ctr[C_MOVE_BEGIN + L] = base;
+    D.ctr[C_MOVE_END + L] = base;
+  }
+  if (l <= 0) return;
+  // allocated prefixes: the rest scores -FLT_MAX and follows in index order
+  const long long nb = min(d0, D.load[L]), nd = min(d1, 8 * D.load[L + 1]);
+  const uint32_t fb = (uint32_t)D.g.off[L], fd = (uint32_t)(8 * D.g.off[L + 1]);
+  auto bkey = [](float s) { return block_key(s); };
+  auto dkey = [](float s) { return dest_key(s); };
+  auto all = [](float) { return true; };
+  const DcList<decltype(bkey), decltype(all)> B{D.bs + fb, nb, fb, bkey, all};
+  const DcList<decltype(dkey), decltype(all)> E{D.ss + fd, nd, fd, dkey, all};
+  u64 bestb = ~0ull, beste = ~0ull;
+  dc_each(B.s, nb, [&](long long i, float v) { bestb = min(bestb, B.full(i, v)); });
+  dc_each(E.s, nd, [&](long long i, float v) { beste = min(beste, E.full(i, v)); });
+  bestb = dc_min(bestb);
+  beste = dc_min(beste);
+  const float sb0 = (bestb >> 32) == 0xFFFFFFFFull ? -1.f : __uint_as_float((uint32_t)(bestb >> 32));
+  const float sd0 = dest_score((uint32_t)(beste >> 32));
+  long long matches = 0;
+  if (nb > 0 && nd > 0 && sb0 >= 0.f && sd0 >= 0.f && sb0 < sd0) {
+    // only these can be in a matched pair; they lead both orders
+    auto bin = [sd0](float s) { return s >= 0.f && s < sd0; };
+    auto din = [sb0](float s) { return s > sb0; };
+    const DcList<decltype(bkey), decltype(bin)> Bc{B.s, nb, fb, bkey, bin};
+    const DcList<decltype(dkey), decltype(din)> Ec{E.s, nd, fd, dkey, din};
+    __syncthreads();
+    if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t c0 = 0, c1 = 0;
+    dc_each(B.s, nb, [&](long long, float v) { c0 += bin(v); });
+    dc_each(E.s, nd, [&](long long, float v) { c1 += din(v); });
+    c0 = __reduce_add_sync(0xffffffffu, c0);
+    c1 = __reduce_add_sync(0xffffffffu, c1);
+    if ((threadIdx.x & 31) == 0) {
+      atomicAdd(&s_cnt[0], c0);
+      atomicAdd(&s_cnt[1], c1);
+    }
+    __syncthreads();
+    const long long top = min(l, min((long long)s_cnt[0], (long long)s_cnt[1]));  // no pair from here on matches
+    long long cb = s_cnt[0], cd = s_cnt[1];
+    u64 ab = 0, ad = 0;
+    bool any = false;
+    while (matches < top) {
+      const int kb = dc_take(Bc, ab, any, cb, top - matches, lb);
+      const int kd = dc_take(Ec, ad, any, cd, top - matches, ld);
+      const int k = min(kb, kd);
+      if (k <= 0) break;  // not reached: top - matches members of both are left
+      __syncthreads();
+      if (threadIdx.x == 0) s_fail = (uint32_t)k;
+      __syncthreads();
+      for (int m = threadIdx.x; m < k; m += DC_THREADS) {
+        const float sb = __uint_as_float((uint32_t)(lb[m] >> 32)), sd = dest_score((uint32_t)(ld[m] >> 32));
+        if (!(sb >= 0.f && sd >= 0.f && sb < sd)) atomicMin(&s_fail, (uint32_t)m);
+      }
+      __syncthreads();
+      const int ok = (int)s_fail;
+      for (int m = threadIdx.x; m < ok; m += DC_THREADS) {
+        D.moves[2 * (base + matches + m)] = (uint32_t)lb[m];
+        D.moves[2 * (base + matches + m) + 1] = (uint32_t)ld[m];
+        if (!D.g.ref_compat || matches + m >= 1) D.bs[(uint32_t)ld[m] >> 3] = -FLT_MAX;
+      }
+      matches += ok;
+      if (ok > 0) {
+        ab = lb[ok - 1];
+        ad = ld[ok - 1];
+        any = true;
+      }
+      __syncthreads();
+      if (ok < k) break;
+      cb -= k;
+      cd -= k;
+    }
+    // ref_compat protects the candidate after the last match too (an
+    // unallocated one is out of the selection as it is)
+    if (D.g.ref_compat && matches >= 1 && matches < d1) {
+      u64 next = ~0ull;
+      dc_each(E.s, nd, [&](long long i, float v) {
+        const u64 k = E.full(i, v);
+        if (k > ad) next = min(next, k);
+      });
+      next = dc_min(next);
+      if (threadIdx.x == 0 && next != ~0ull) D.bs[(uint32_t)next >> 3] = -FLT_MAX;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    D.move_limit[L] = (long long)(u64)((float)matches * 1.2f);
+    D.ctr[C_MATCHES] = matches;
+    D.ctr[C_MOVES] = base + matches;
+    D.ctr[C_MOVE_END + L] = base + matches;
+  }
+  __syncthreads();
+}
+
+// stable compaction of the subblocks of level L that flag(score, index) picks:
+// their number; every thread takes a block's eight subblocks at a time
+template <class Flag> __device__ __forceinline__ uint32_t dc_compact(const Dev &D, int L, long long nblk, Flag flag, uint32_t *out) {
+  uint32_t run = 0;
+  const long long first = D.g.off[L];
+  for (long long t0 = 0; t0 < nblk; t0 += DC_THREADS) {
+    const long long t = t0 + threadIdx.x;
+    unsigned f = 0;
+    const uint32_t sb = (uint32_t)(8 * (first + t));
+    if (t < nblk) {
+      const float4 a = reinterpret_cast<const float4 *>(D.ss + sb)[0], b = reinterpret_cast<const float4 *>(D.ss + sb)[1];
+      const float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int k = 0; k < 8; k++) f |= (flag(v[k], sb + k) ? 1u : 0u) << k;
+    }
+    uint32_t total;
+    uint32_t at = run + dc_scan((uint32_t)__popc(f), &total);
+    for (int k = 0; k < 8; k++)
+      if ((f >> k) & 1u) out[at++] = sb + k;
+    run += total;
+  }
+  __syncthreads();
+  return run;
+}
+// the refinements of one parent level (refine_setup to record_refines above)
+__device__ __forceinline__ void dc_refines(const Dev &D, int L, uint32_t *cand) {
+  const u64 a = (u64)(D.g.budget[L - 1] - D.load[L - 1]), bb = (u64)(8 * D.load[L]) - (u64)D.load[L - 1];
+  const long long limit = (long long)(a < bb ? a : bb);
+  const long long base = D.ctr[C_REFINES], load0 = D.load[L - 1];
+  __syncthreads();
+  long long keep = 0;
+  if (limit != 0) {
+    const float thr = D.ph.refine_threshold;
+    // unallocated blocks score -FLT_MAX
+    const long long nblk = thr < -FLT_MAX ? D.g.budget[L] : min(D.g.budget[L], D.load[L]);
+    uint32_t n = dc_compact(D, L, nblk, [thr](float s, uint32_t) { return s > thr; }, cand);
+    keep = (long long)n < limit ? (long long)n : limit;
+    long long from = 0;
+    if (D.g.ref_compat) {
+      from = (long long)n - keep;  // the largest indices
+    } else if ((long long)n > limit) {  // the best scores, in index order
+      auto dkey = [](float s) { return dest_key(s); };
+      auto in = [thr](float s) { return s > thr; };
+      const uint32_t fd = (uint32_t)(8 * D.g.off[L]);
+      const DcList<decltype(dkey), decltype(in)> E{D.ss + fd, 8 * nblk, fd, dkey, in};
+      const u64 worst = dc_select(E, 0, false, (uint32_t)limit);
+      n = dc_compact(D, L, nblk,
+                     [thr, worst](float s, uint32_t i) { return s > thr && (((u64)dest_key(s) << 32) | i) <= worst; }, cand);
+    }
+    for (long long r = threadIdx.x; r < keep; r += DC_THREADS) {
+      D.refines[2 * (base + r)] = cand[from + r];
+      D.refines[2 * (base + r) + 1] = (uint32_t)(D.g.off[L - 1] + load0 + r);
+    }
+  }
+  if (threadIdx.x == 0) {
+    D.ctr[C_REF_BEGIN + L - 1] = base;
+    D.ctr[C_REF_END + L - 1] = base + keep;
+    D.ctr[C_LOAD0 + L - 1] = load0;
+    D.ctr[C_REFINES] = base + keep;
+  }
+  __syncthreads();
+}
+static __host__ __device__ bool decide_full(const Geom &g, int L) { return g.budget[L] == g.full[L]; }
+
+// PHASE 0: the moves of every level and their application, coarse to fine;
+// 1: the refinements, their application and the loads. One CTA per member.
+struct DecideP {
+  int n;
+  uint32_t *prevs[BMAX], *cand[BMAX];
+  Dev d[BMAX];
+};
+static_assert(sizeof(DecideP) < 32000, "kernel parameter space");
+template <int PHASE> __global__ void __launch_bounds__(DC_THREADS, 1) k_decide(const __grid_constant__ DecideP P) {
+  extern __shared__ __align__(16) u64 dc_lists[];
+  const Dev &D = P.d[blockIdx.x];
+  if (PHASE == 0) {
+    for (int L = 0; L < D.g.levels - 1; L++)
+      if (!decide_full(D.g, L)) dc_moves(D, L, dc_lists, dc_lists + DC_LIST);
+    __syncthreads();
+    for (int L = D.g.levels - 2; L >= 0; L--) {
+      if (!decide_full(D.g, L)) apply_moves_body(D, L, P.prevs[blockIdx.x], 0, 1);
+      __syncthreads();
+    }
+  } else {
+    for (int L = 1; L < D.g.levels; L++)
+      if (!decide_full(D.g, L - 1)) dc_refines(D, L, P.cand[blockIdx.x]);
+    __syncthreads();
+    apply_refines_body(D, 0, 1);
+    __syncthreads();
+    if (threadIdx.x == 0) finish_refines_body(D, 0, 1);
+  }
+}
+static void launch_decide(int phase, const DecideP &P, cudaStream_t st) {
+  if (phase == 0) {
+    static const cudaError_t ok = cudaFuncSetAttribute(k_decide<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SMEM);
+    (void)ok;
+    k_decide<0><<<P.n, DC_THREADS, DC_SMEM, st>>>(P);
+  } else {
+    k_decide<1><<<P.n, DC_THREADS, 0, st>>>(P);
+  }
+}
+
 static unsigned grid_for(long long n, int threads = 256) {
   return (unsigned)((n + threads - 1) / threads);
 }
@@ -704,11 +1092,25 @@ static bool level_full(const Geom &g, int L) { return g.budget[L] == g.full[L]; 
 void launch_adapt(const Dev &D, const SortScratch &s, uint32_t *keys, uint32_t *vals, uint32_t *keys2,
                   uint32_t *vals2, int sms, cudaStream_t st) {
   const unsigned gs = (unsigned)(sms > 0 ? sms * 4 : 512);
-  cudaMemsetAsync(D.ctr, 0, sizeof(long long) * C_COUNT, st);
-  cudaMemsetAsync(D.flags, 0, (size_t)D.g.B, st);
   // moveBlocks
   launch_scores(D, st);
-  k_block_scores<<<grid_for(D.g.B), 256, 0, st>>>(D);
+  k_block_scores<<<grid_for(std::max<long long>(D.g.B, C_COUNT)), 256, 0, st>>>(D);
+  if (D.g.B <= kDecideBlocks) {
+    DecideP P{};
+    P.n = 1;
+    P.d[0] = D;
+    P.prevs[0] = keys;
+    P.cand[0] = vals;
+    const bool any = D.g.sparse > 0;  // some level is not full: there is something to decide
+    if (any) {
+      launch_decide(0, P, st);
+      k_rescore<<<gs, 256, 0, st>>>(D, keys);
+      launch_decide(1, P, st);
+    }
+    k_refresh_nbr<<<grid_for(D.g.B * 27), 256, 0, st>>>(D);
+    for (int L = D.g.levels - 2; L >= 0; L--) k_propagate<<<gs, 256, 0, st>>>(D, L);
+    return;
+  }
   for (int L = 0; L < D.g.levels - 1; L++) {
     if (level_full(D.g, L)) continue;  // no free place at level L: no move (limit 0)
     const long long d0 = D.g.budget[L], d1 = 8 * D.g.budget[L + 1];
@@ -932,7 +1334,7 @@ static void launch_scores_staged(const Dev *d, int n, cudaStream_t st) {
 // member without the launch's level (or of the other selection mode) gets no
 // CTAs. The bodies are the single simulation's, so the results are too.
 enum : int {
-  A_CLEAR, A_SCORES, A_BLOCK_SCORES, A_MOVE_SETUP, A_KEYS, A_MATCH, A_COMMIT, A_APPLY_MOVES, A_REFINE_SETUP,
+  A_SCORES, A_BLOCK_SCORES, A_MOVE_SETUP, A_KEYS, A_MATCH, A_COMMIT, A_APPLY_MOVES, A_REFINE_SETUP,
   A_CMP_COUNT, A_CMP_SCAN, A_CMP_SCATTER, A_RECORD, A_KEYS_CANDS, A_CLEAR_SEL, A_MARK, A_APPLY_REFINES,
   A_FINISH, A_NBR, A_PROPAGATE, A_RESCORE
 };
@@ -946,15 +1348,6 @@ struct AdaptBatchP {
 };
 static_assert(sizeof(AdaptBatchP) < 32000, "kernel parameter space");
 
-// clears the counters and the block flags of one member
-__device__ __forceinline__ void clear_body(const Dev &D, unsigned bx, unsigned gx) {
-  const long long n = D.g.B > C_COUNT ? D.g.B : C_COUNT;
-  for (long long i = (long long)bx * blockDim.x + threadIdx.x; i < n; i += (long long)gx * blockDim.x) {
-    if (i < C_COUNT) D.ctr[i] = 0;
-    if (i < D.g.B) D.flags[i] = 0;
-  }
-}
-
 template <int OP, int T> __global__ void __launch_bounds__(T) k_adapt_batch(const __grid_constant__ AdaptBatchP P) {
   int s = 0;
   while (s < P.n - 1 && blockIdx.x >= P.end[s]) s++;
@@ -962,7 +1355,6 @@ template <int OP, int T> __global__ void __launch_bounds__(T) k_adapt_batch(cons
   const unsigned bx = (unsigned)(blockIdx.x - first), gx = (unsigned)(P.end[s] - first);
   const Dev &D = P.d[s];
   const int L = P.L;
-  if constexpr (OP == A_CLEAR) clear_body(D, bx, gx);
   if constexpr (OP == A_SCORES) {
     if (D.ph.criterion == 0)
       scores_geo_body(D, bx, gx);
@@ -1062,10 +1454,30 @@ struct AdaptLauncher {
   void run() {
     int maxl = 0;
     for (int i = 0; i < n; i++) maxl = std::max(maxl, levels(i));
-    go<A_CLEAR>([&](int i) { return (long long)std::min<long long>(gs, grid_for(std::max<long long>(B(i), C_COUNT))); });
     // moveBlocks
     scores();
-    go<A_BLOCK_SCORES>([&](int i) { return (long long)grid_for(B(i)); });
+    go<A_BLOCK_SCORES>([&](int i) { return (long long)grid_for(std::max<long long>(B(i), C_COUNT)); });
+    bool small = true, any = false;
+    for (int i = 0; i < n; i++) {
+      small = small && B(i) <= kDecideBlocks;
+      any = any || m[i].D.g.sparse > 0;
+    }
+    if (small) {
+      DecideP Q{};
+      Q.n = n;
+      for (int i = 0; i < n; i++) {
+        Q.d[i] = m[i].D;
+        Q.prevs[i] = P.p0[i] = m[i].keys;
+        Q.cand[i] = m[i].vals;
+      }
+      if (any) {
+        launch_decide(0, Q, st);
+        go<A_RESCORE>([&](int i) { return gs; });
+        launch_decide(1, Q, st);
+      }
+      refresh(maxl);
+      return;
+    }
     for (int L = 0; L < maxl - 1; L++) {
       P.L = L;
       auto has = [&](int i) { return L < levels(i) - 1 && !level_full(m[i].D.g, L); };
@@ -1154,7 +1566,10 @@ struct AdaptLauncher {
     }
     go<A_APPLY_REFINES>([&](int i) { return gs; });
     go<A_FINISH, 32>([&](int i) { return 1; });
-    // neighbour tables + value propagation for touched blocks
+    refresh(maxl);
+  }
+  // neighbour tables + value propagation for touched blocks
+  void refresh(int maxl) {
     go<A_NBR>([&](int i) { return (long long)grid_for(B(i) * 27); });
     for (int L = maxl - 2; L >= 0; L--) {
       P.L = L;

@@ -122,3 +122,39 @@ def test_uniform_sweeps_bitexact(size, iters, compat):
         for f in ("pressure", "pressure_tmp", "divergence", "vel_x", "vel_y", "vel_z", "density"):
             a, b = g.get_field(f), o.get_field(f).astype(np.float32)
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32)), f"{f}: {(a != b).sum()} cells differ"
+
+
+# Adaptation decisions on long lists: more refinement candidates than free
+# blocks, then a flow that leaves one half of the domain for the other, so that
+# thousands of blocks move at once (more than one list of the selection holds)
+@pytest.mark.parametrize("compat", [0, 1])
+@pytest.mark.parametrize("blocks", [300, 9000])
+def test_many_moves_and_refinements(blocks, compat):
+    p = scenarios.plume(128, 128, 128, 4096 + blocks, 2, 2)
+    p.refine_criterion = capi.REFINE_FIELDS
+    p.refine_threshold, p.vort_threshold, p.grad_threshold = 1e-6, 0.5, 0.05
+    p.ref_compat = compat
+    g, o = pair(p, 0.0)
+    rng = np.random.default_rng(blocks + compat)
+    most = 0
+    for half in (0, 1, 0, 0):
+        topo = o.get_topology()
+        scale = 2.0 ** np.maximum(topo["pos"][:, 3], 0)
+        far = (topo["pos"][:, 0] * scale >= 64) == bool(half)
+        amp = np.repeat(np.where(far, 1.0, 1e-3), 64).astype(np.float32)
+        for f in ("vel_x", "vel_y", "vel_z"):
+            v = amp * rng.standard_normal(g.num_cells).astype(np.float32)
+            g.set_field(f, v)
+            o.set_field(f, v)
+        g.adapt()
+        o.adapt()
+        g.sync()
+        (mg, rg), (mo, ro) = g.get_last_adapt(), o.get_last_adapt()
+        assert np.array_equal(mg, mo) and np.array_equal(rg, ro)
+        tg, to = g.get_topology(), o.get_topology()
+        alloc = to["pos"][:, 3] >= 0
+        assert np.array_equal(tg["pos"][alloc], to["pos"][alloc])
+        for k in ("load", "move_limit"):
+            assert np.array_equal(tg[k], to[k])
+        most = max(most, len(mo))
+    print("largest number of moves:", most)
