@@ -251,8 +251,8 @@ struct UDev {
 void launch_u_fluidity(const UDev &U, cudaStream_t st);
 void launch_u_sources(const UDev &U, cudaStream_t st);
 void launch_u_advect_velocity(const UDev &U, cudaStream_t st);
-void launch_u_advect_scalars(const UDev &U, cudaStream_t st);
-void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, int sms, cudaStream_t st);
+void launch_u_advect_scalars(const UDev &U, bool apply, cudaStream_t st);  // apply: the pressure application first
+void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, bool apply, int sms, cudaStream_t st);
 void launch_u_add_noise(const UDev &U, unsigned long long seed, float amp, cudaStream_t st);
 void launch_u_stats(const UDev &U, cudaStream_t st);
 void launch_render_adaptive(const Dev &D, const RenderP &R, float4 *out, cudaStream_t st);

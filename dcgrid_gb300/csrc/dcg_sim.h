@@ -754,13 +754,13 @@ struct dcg_sim {
     vpar ^= 1;
     bind_parity();
   }
-  void u_project(bool local) {
+  void u_project(bool local, bool apply = true) {
     const int top_pairs = P.ref_compat ? 2 : P.jacobi_iters / 2;
     const int pairs = local ? (P.ref_compat ? 5 : P.jacobi_iters / 2) : (P.ref_compat ? 1 : P.jacobi_iters / 2);
-    launch_u_project(U, top_pairs, pairs, local, sms, stream);
+    launch_u_project(U, top_pairs, pairs, local, apply, sms, stream);
   }
-  void u_advect_scalars() {
-    launch_u_advect_scalars(U, stream);
+  void u_advect_scalars(bool apply = false) {
+    launch_u_advect_scalars(U, apply, stream);
     qpar ^= 1;
     bind_parity();
   }
@@ -787,8 +787,8 @@ struct dcg_sim {
       a_project(false, false);
       a_apply_advect();
     } else {
-      stage_project(false);
-      stage_advect_scalars();
+      u_project(false, false);
+      u_advect_scalars(true);  // with the pressure application in the same pass
     }
   }
 
