@@ -90,7 +90,7 @@ struct dcg_batch {
 
   int set_solve_config() {
     if (tune.solve_barrier < 0 || tune.solve_barrier > 7)
-      return fail(DCG_E_INVALID, "solve_barrier must be 0..7 (bit 0: two-level barrier)");
+      return fail(DCG_E_INVALID, "solve_barrier must be 0..7");
     if (!solve_variant_valid(tune.solve_cache))
       return fail(DCG_E_INVALID, "solve_cache must be 0, 3, 4, 8 or a pipelined variant 16, 18, 19, 32, 34, 35, 64, 66, 83");
     for (int k = 0; k < 4; k++)
@@ -187,15 +187,13 @@ struct dcg_batch {
   }
   // the cascade with the tuned schedule of each round of the general solve
   void solve_tuned() {
-    solve([&](int round, int &grid, int &cache, int &tree) {
+    solve([&](int round, int &grid, int &cache) {
       if (round < 4 && tune.round_ctas_per_sm[round] != 0) {
         cache = tune.round_cache[round];
         grid = batch_solve_grid(sms, cache, tune.round_ctas_per_sm[round]);
-        tree = tune.round_barrier[round];
       } else {
         grid = solve_grid;
         cache = tune.solve_cache;
-        tree = tune.solve_barrier & 1;
       }
     });
   }
@@ -217,8 +215,8 @@ struct dcg_batch {
     c.sweeps = iters;
     c.st = stream;
     c.run(d.data(), raster.data(), n(), [&](const std::vector<int> &mem, const std::vector<int> &lev, long long limit, int round) {
-      int grid = 0, cache = 0, tree = 0;
-      schedule(round, grid, cache, tree);
+      int grid = 0, cache = 0;
+      schedule(round, grid, cache);
       for (size_t g = 0; g < mem.size(); g += BMAX) {
         SolveBatch P{};
         P.n = (int)std::min<size_t>(BMAX, mem.size() - g);
@@ -235,7 +233,7 @@ struct dcg_batch {
           P.lev[i] = lev[g + i];
           P.cl_max[i] = limit;
         }
-        launch_level_solve_batch(P, iters, grid, cache, tree, stream);
+        launch_level_solve_batch(P, iters, grid, cache, stream);
       }
     });
   }
@@ -466,28 +464,25 @@ struct dcg_batch {
       best.cells_ms[stage] = ms_of[pick][stage];
     }
     // the general level solve (levels that no cluster holds): cache depth x
-    // CTAs per SM x barrier kind, timed with the whole cascade
+    // CTAs per SM, timed with the whole cascade
     float best_solve = 1e30f;
     for (int r = 0; r < 4; r++) best.round_ctas_per_sm[r] = 0;
     for (int cache : {0, 3, 4, 8, 16, 18, 19, 32, 34, 35, 64, 66, 83}) {
       const int occ = batch_solve_grid(sms, cache, 0) / std::max(1, sms);
-      for (int k = 1; k <= occ; k++)
-        for (int tb = 0; tb < 2; tb++) {  // two-level barrier
-          const int grid = batch_solve_grid(sms, cache, k);
-          const float ms = time_ms(reps, [&] {
-            solve([&](int, int &g, int &c, int &t) {
-              g = grid;
-              c = cache;
-              t = tb;
-            });
+      for (int k = 1; k <= occ; k++) {
+        const int grid = batch_solve_grid(sms, cache, k);
+        const float ms = time_ms(reps, [&] {
+          solve([&](int, int &g, int &c) {
+            g = grid;
+            c = cache;
           });
-          if (ms < best_solve) {
-            best_solve = ms;
-            best.solve_cache = cache;
-            best.solve_ctas_per_sm = k;
-            best.solve_barrier = tb;
-          }
+        });
+        if (ms < best_solve) {
+          best_solve = ms;
+          best.solve_cache = cache;
+          best.solve_ctas_per_sm = k;
         }
+      }
     }
     best.solve_ms = best_solve;
     if ((rc = sync())) return rc;

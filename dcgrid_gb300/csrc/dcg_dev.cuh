@@ -99,17 +99,15 @@ struct Dev {
   long long *ctr;          // C_COUNT counters
   uint32_t *err;           // device error word
   double *red;             // reductions (stats)
-  uint32_t *bar;           // grid barrier {arrivals, generation}
-  uint32_t *epoch;         // per block: sweeps completed in the running level solve
+  uint32_t *bar;           // grid barrier (GridBarrier)
   uint32_t *binfo;         // level solve: block descriptions of the running level (BI_WORDS words per block)
   float *rr, *e, *et;      // defect correction: residual, correction and its ping-pong plane
   double *dnorm;           // defect correction: FP64 ||r||^2, ||div||^2 per pass
 };
 
-// Scoped atomics of the grid barriers (PTX memory model): arrivals are
-// acquire-release read-modify-writes, the release of the waiting CTAs a
-// release add on the generation word, the wait an acquire load of it. Before
-// the arrival, __syncthreads orders the CTA's writes before thread 0's release;
+// Scoped atomics of the grid barrier (PTX memory model): an arrival is a
+// release (or acquire-release) add, the wait an acquire load of the same word,
+// and the adds in between continue the release sequence. Before the arrival, __syncthreads orders the CTA's writes before thread 0's release;
 // after the wait, __syncthreads orders thread 0's acquire before the CTA's
 // reads; so every write before the barrier is visible to every read after it.
 __device__ __forceinline__ unsigned atom_add_acq_rel(unsigned *p, unsigned v) {
@@ -125,80 +123,50 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p) {
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_relaxed(unsigned *p, unsigned v) {
-  asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-// Bounded wait for the generation word to leave g: after `limit` polls (2^22
-// by default) the CTA records DCG_DEVERR_TIMEOUT (8) in the error word and
-// gives up.
+// Polls of a bounded wait before it gives up.
 constexpr unsigned kPollLimit = 1u << 22;
-__device__ __forceinline__ void barrier_wait(const unsigned *gen, unsigned g, uint32_t *errw,
-                                             unsigned limit = kPollLimit) {
-  volatile unsigned *err = errw;
-  unsigned spins = 0;
-  while (ld_acquire(gen) == g) {
-    __nanosleep(32);
-    if (++spins > limit || (*err & 8u)) {
-      atomicOr(errw, 8u);
-      break;
-    }
-  }
-}
 
-// Two-level grid barrier: CTAs arrive on one of 16 group counters (separate
-// 128-byte lines); the last of each group arrives on the top counter, and the
-// last there releases everyone through the generation word. Same bounded wait
-// and timeout rule as grid_barrier. Layout (u32, from bar + 64): [0]
-// generation, [32*(1+g)] group g counter, [32*17] top counter.
-__device__ inline void grid_barrier_tree(uint32_t *bar, uint32_t *errw, unsigned nctas) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned *tb = bar + 64;
-    volatile unsigned *err = errw;
-    if ((*err & 8u) == 0) {
-      const unsigned g = ld_acquire(tb);
-      const unsigned grp = blockIdx.x & 15u;
-      const unsigned members = (nctas >> 4) + ((grp < (nctas & 15u)) ? 1u : 0u);
-      const unsigned groups = nctas < 16u ? nctas : 16u;
-      bool release = false;
-      if (atom_add_acq_rel(tb + 32 * (1 + grp), 1u) == members - 1) {
-        st_relaxed(tb + 32 * (1 + grp), 0u);
-        if (atom_add_acq_rel(tb + 32 * 17, 1u) == groups - 1) {
-          st_relaxed(tb + 32 * 17, 0u);
-          release = true;
+// Grid-wide barrier for cooperative launches (all CTAs co-resident), one object
+// per CTA and launch. One word counts the arrivals: CTA 0 adds 2^31 - (n - 1),
+// the others 1, so the sum of n arrivals flips the word's top bit and leaves
+// the rest at zero; a CTA waits for the flip. A launch's first arrival learns
+// the phase of the top bit from the value that its atomic returns; every later
+// one needs no answer and is a release reduction. The wait is bounded: after
+// `limit` polls the CTA records DCG_DEVERR_TIMEOUT (8) in the error word and
+// continues; once that bit is set a barrier that finds its CTAs missing
+// returns at once, so a broken barrier costs one bounded wait and never hangs
+// the GPU. What bounds it is the chain of L2 round trips: the CTA's stores
+// performed, the reduction, the poll. A generation word read before the
+// arrival, an error word read before that and a separate release word made it
+// five round trips, a tree of group counters six: a sweep of 4096 blocks took
+// 4.6 us with the tree and takes 3.1, one of 8192 blocks 5.3 and 3.9.
+struct GridBarrier {
+  uint32_t *word, *err;
+  unsigned n, phase;
+  bool known;
+  __device__ GridBarrier(uint32_t *w, uint32_t *e, unsigned nctas) : word(w), err(e), n(nctas), phase(0u), known(false) {}
+  __device__ void sync(unsigned limit = kPollLimit) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const unsigned inc = blockIdx.x == 0 ? 0x80000000u - (n - 1) : 1u;
+      if (known) {
+        red_add_release(word, inc);
+      } else {
+        phase = atom_add_acq_rel(word, inc) & 0x80000000u;
+        known = true;
+      }
+      unsigned spins = 0;
+      while ((ld_acquire(word) & 0x80000000u) == phase) {
+        if (++spins > limit || (*(volatile uint32_t *)err & 8u)) {
+          atomicOr(err, 8u);
+          break;
         }
       }
-      if (release)
-        red_add_release(tb, 1u);
-      else
-        barrier_wait(tb, g, errw);
+      phase ^= 0x80000000u;
     }
+    __syncthreads();
   }
-  __syncthreads();
-}
-__device__ inline void grid_barrier_tree(const Dev &D, unsigned nctas) { grid_barrier_tree(D.bar, D.err, nctas); }
-
-// Grid-wide barrier for cooperative launches (all CTAs co-resident). The wait
-// is bounded: after 2^22 polls the CTA records DCG_DEVERR_TIMEOUT (8) in the
-// error word and continues; once that bit is set every later barrier returns
-// at once, so a broken barrier costs one bounded wait and never hangs the GPU.
-__device__ inline void grid_barrier(uint32_t *bar, uint32_t *errw, unsigned nctas, unsigned limit = kPollLimit) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned *err = errw;
-    if ((*err & 8u) == 0) {
-      const unsigned g = ld_acquire(bar + 1);
-      if (atom_add_acq_rel(bar, 1u) == nctas - 1) {
-        st_relaxed(bar, 0u);
-        red_add_release(bar + 1, 1u);
-      } else {
-        barrier_wait(bar + 1, g, errw, limit);
-      }
-    }
-  }
-  __syncthreads();
-}
-__device__ inline void grid_barrier(const Dev &D, unsigned nctas) { grid_barrier(D.bar, D.err, nctas); }
+};
 
 // ---------------------------------------------------------------- index math
 __host__ __device__ inline int spread2(int d, int off) { return ((d & 1) | ((d << 2) & 8)) << off; }

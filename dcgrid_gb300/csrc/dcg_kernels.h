@@ -52,7 +52,7 @@ void launch_apply_pressure(const Dev &D, cudaStream_t st);
 void launch_add_correction(const Dev &D, cudaStream_t st);
 // cooperative persistent solve of one level (prolongation + sweeps)
 int level_solve_grid(int sms);
-void launch_level_solve(const Dev &D, int level, int prolong, int sweeps, int grid, int epoch_sync, cudaStream_t st);
+void launch_level_solve(const Dev &D, int level, int prolong, int sweeps, int grid, cudaStream_t st);
 
 // ---- batched launches (many independent simulations per launch)
 // Member devices travel in the kernel parameters (__grid_constant__, read
@@ -119,7 +119,7 @@ void launch_add_correction_batch(CellBatch &P, cudaStream_t st);
 // and CTAs per SM (0 = occupancy limit)
 int batch_solve_grid(int sms, int cache, int ctas_per_sm);
 bool solve_variant_valid(int cache);
-void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cache, int tree, cudaStream_t st);
+void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cache, cudaStream_t st);
 
 // k_cascade.cu: cluster size of the device's cluster solve (0: none), blocks a
 // cluster of that size holds, and the launch (it picks P.csize)
@@ -176,9 +176,9 @@ struct Cascade {
   int sms = 148;
   int sweeps = 0, prolong = 1;
   cudaStream_t st = nullptr;
-  // blocks that make the dense solve the faster one (a box of 8192 blocks: 6.9
-  // us per sweep, grid-wide 5.3; of 32768: 8.3 and 9.3)
-  static constexpr long long kDenseBlocks = 16384;
+  // blocks that make the dense solve the faster one (a box of 32768 blocks: 8.3
+  // us per sweep, grid-wide 7.7; of 65536: 8.5 and 13.0)
+  static constexpr long long kDenseBlocks = 36864;
   long long limit() const { return csize > 0 ? cluster_solve_blocks(csize) : 0; }
   // general(members, levels, limit, round): solve levels[i] of members[i]
   // unless at most `limit` of its blocks are allocated

@@ -139,11 +139,9 @@ struct dcg_sim {
   bool use_graphs = true;
   long long kernels_per_step = 0;
   int ls_grid = 0;  // CTAs of the cooperative level solve (0 = per-sweep launches)
-  // level solve kernel: 3 = the staged solve shared with batches (two-level
-  // barrier); 2 = the per-level kernel with a two-level barrier, taken when
-  // the staged solve's cooperative grid cannot be formed on the device
-  int ls_epoch = 3;
-  int ls_grid_staged = 0;  // CTAs of the staged solve
+  // CTAs of the staged solve shared with batches (0: its cooperative grid
+  // cannot be formed on the device, and the per-level kernel takes its place)
+  int ls_grid_staged = 0;
   int cl_size = 0;         // cluster size of the small levels' solve (0: none)
   // the full levels lie in raster order, as created (a caller's topology or
   // state may say otherwise: check_raster)
@@ -370,7 +368,6 @@ struct dcg_sim {
     if ((rc = alloc(&D.err, 4))) return rc;
     if ((rc = alloc(&D.red, 32))) return rc;
     if ((rc = alloc(&D.bar, 64 + 32 * 18))) return rc;
-    if ((rc = alloc(&D.epoch, B))) return rc;
     if ((rc = alloc(&D.binfo, (long long)BI_WORDS * B))) return rc;
     if (P.defect_passes > 0) {
       if (ext_rr) {
@@ -388,7 +385,6 @@ struct dcg_sim {
     if (plan_only) return plan_tail_adaptive(B);
     ls_grid = level_solve_grid(sms);
     ls_grid_staged = batch_solve_grid(sms, kSolveVariant, 0);
-    if (ls_grid_staged <= 0 && ls_epoch == 3) ls_epoch = 2;
     cl_size = cluster_solve_size();
     if (P.emission_n > 0) {
       const size_t ne = (size_t)P.emission_n * P.emission_n * P.emission_n;
@@ -531,12 +527,12 @@ struct dcg_sim {
       // one cooperative launch per level: prolongation (not for the coarsest
       // level, nor in projectLocal) and all of the level's sweeps
       const int sweeps = local ? 2 * P.jacobi_iters : P.jacobi_iters;
-      if (ls_epoch == 3) {
+      if (ls_grid_staged > 0) {
         solve_cascade(local ? 0 : 1, sweeps);
         if (!local && P.defect_passes > 0) defect_correct(sweeps);
       } else {
         for (int l = top; l >= 0; l--)
-          launch_level_solve(D, l, (!local && l < top) ? 1 : 0, sweeps, ls_grid, ls_epoch, stream);
+          launch_level_solve(D, l, (!local && l < top) ? 1 : 0, sweeps, ls_grid, stream);
       }
     } else if (local) {
       const int pairs = P.jacobi_iters;
@@ -652,7 +648,7 @@ struct dcg_sim {
     SB.lev[0] = level;
     SB.cl_max[0] = limit;
     SB.d[0] = d;
-    launch_level_solve_batch(SB, sweeps, ls_grid_staged, kSolveVariant, 1, stream);
+    launch_level_solve_batch(SB, sweeps, ls_grid_staged, kSolveVariant, stream);
   }
   void a_advect_scalars() {
     cells(1, 1);

@@ -305,78 +305,22 @@ __device__ inline float jacobi_update(const float *src, const Nb6 &n, float ad) 
               __ldcg(src + n.i4) + __ldcg(src + n.i5) - ad);
 }
 
-__device__ inline uint32_t ld_acquire_u32(const uint32_t *p) {
-  uint32_t v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-__device__ inline void st_release_u32(uint32_t *p, uint32_t v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Neighbour epochs: epoch[b] = sweeps block b has completed in the current
-// level solve. Before sweep k (1-based) of a CTA's blocks, their same-level
-// face neighbours must have completed sweep k-1: then the values read are
-// current and nobody still reads the buffer being written. Coarser neighbours
-// are constant during the solve and need no wait. Thread i < 24*rounds polls
-// face i%6 of block i/6 of the CTA; the wait is bounded (2^22 polls) and
-// records DCG_DEVERR_TIMEOUT (8) when exceeded. Writes are ordered before the
-// release store by bar.sync; the acquire load orders later reads the same way.
-__device__ inline long long cta_block(long long off, int j, unsigned nctas) {
-  return off + 4 * ((long long)(j >> 2) * nctas + blockIdx.x) + (j & 3);
-}
-__device__ inline void wait_neighbours(const Dev &D, long long off, long long blk_end, int rounds, unsigned nctas,
-                                       uint32_t need) {
-  const int t = threadIdx.x;
-  if (need > 0 && t < 24 * rounds) {
-    const long long b = cta_block(off, t / 6, nctas);
-    if (b < blk_end) {
-      const int f = t % 6;
-      const int dir = f == 0 ? 4 : f == 1 ? 22 : f == 2 ? 10 : f == 3 ? 16 : f == 4 ? 12 : 14;
-      const uint32_t e = D.nbr[27 * b + dir];
-      if (e != OUT && (e >> 28) == 0 && (e & NBR_MASK) != (uint32_t)b) {
-        const uint32_t *ep = D.epoch + (e & NBR_MASK);
-        unsigned spins = 0;
-        while (ld_acquire_u32(ep) < need) {
-          if (++spins > (1u << 22) || (*(volatile uint32_t *)D.err & 8u)) {
-            atomicOr(D.err, 8u);
-            break;
-          }
-          __nanosleep(20);
-        }
-      }
-    }
-  }
-  __syncthreads();
-}
-__device__ inline void publish_blocks(const Dev &D, long long off, long long blk_end, int rounds, unsigned nctas,
-                                      uint32_t done) {
-  __syncthreads();
-  const int t = threadIdx.x;
-  if (t < 4 * rounds) {
-    const long long b = cta_block(off, t, nctas);
-    if (b < blk_end) st_release_u32(D.epoch + b, done);
-  }
-}
-
 constexpr int LS_CACHE = 4;
 
 // The solve of one level of the cascade (fluid_simulation_dcgrid.cu:281-290)
 // in one cooperative launch: optional prolongation from the parent level, then
 // `sweeps` Jacobi sweeps (ping-pong p -> p~ -> p, as k_dcgrid_jacobi/_inv).
 // Work split: CTA c owns the level's blocks 4*(r*grid + c) .. +3 in round r.
-// One grid barrier follows prolongation and the epoch reset; sweeps are then
-// separated by a flat (epoch_sync 0) or two-level (2) grid barrier, or ordered
-// block by block through neighbour epochs (1). The library uses this kernel
-// only where the staged solve (k_level_solve_batch) cannot form its
-// cooperative grid, with the two-level barrier.
+// Grid barriers follow the prolongation and separate the sweeps. The library
+// uses this kernel only where the staged solve (k_level_solve_batch) cannot
+// form its cooperative grid.
 // The level's topology is fixed during the solve, so each thread resolves the
 // six neighbour cells of its (at most LS_CACHE) cells once and keeps them and
 // alpha*div in registers; a sweep is then six loads and one store per cell.
 // Levels with more cells than the grid covers in LS_CACHE rounds resolve
 // neighbours in every sweep. Arithmetic is that of k_jacobi (identical results).
 template <int CACHE>
-__global__ void __launch_bounds__(256) k_level_solve(Dev D, int level, int prolong, int sweeps, int epoch_sync) {
+__global__ void __launch_bounds__(256) k_level_solve(Dev D, int level, int prolong, int sweeps) {
   const unsigned nctas = gridDim.x;
   const long long nblk = D.load[level];
   const long long ncell = nblk * 64;
@@ -387,17 +331,11 @@ __global__ void __launch_bounds__(256) k_level_solve(Dev D, int level, int prolo
   const int rounds = (int)((ncell + stride - 1) / stride);
   const int s = 1 << level;
   const float alpha = (float)(s * s) * D.ph.dx * D.ph.dx;
-  for (long long b = first; b < nblk; b += stride) D.epoch[off + b] = 0u;
   if (prolong)
     for (long long lc = first; lc < ncell; lc += stride) prolong_cell(D, base + lc);
   if (sweeps <= 0) return;
-  // epoch_sync: 0 = flat grid barrier, 1 = neighbour epochs, 2 = two-level barrier
-  auto barrier = [&]() {
-    if (epoch_sync == 2) grid_barrier_tree(D, nctas);
-    else grid_barrier(D, nctas);
-  };
-  barrier();
-  const long long blk_end = off + nblk;
+  GridBarrier bar(D.bar, D.err, nctas);
+  bar.sync();
   if (CACHE > 0 && rounds <= CACHE) {
     // neighbour indices and alpha*div of the thread's cells, [round][k][thread]
     __shared__ uint32_t s_nb[CACHE > 0 ? CACHE : 1][6][256];
@@ -415,7 +353,6 @@ __global__ void __launch_bounds__(256) k_level_solve(Dev D, int level, int prolo
     for (int it = 0; it < sweeps; it++) {
       const float *src = (it & 1) ? D.pt : D.p;
       float *dst = (it & 1) ? D.p : D.pt;
-      if (epoch_sync == 1) wait_neighbours(D, off, blk_end, rounds, nctas, (uint32_t)it);
       for (int r = 0; r < rounds; r++) {
         const long long lc = first + r * stride;
         if (lc < ncell) {
@@ -423,18 +360,16 @@ __global__ void __launch_bounds__(256) k_level_solve(Dev D, int level, int prolo
           dst[base + lc] = jacobi_update(src, n, s_ad[r][t]);
         }
       }
-      if (epoch_sync == 1) publish_blocks(D, off, blk_end, rounds, nctas, (uint32_t)it + 1);
-      else if (it + 1 < sweeps) barrier();
+      if (it + 1 < sweeps) bar.sync();
     }
   } else {
-    // too many rounds for the caches: neighbours resolved every sweep, and a
-    // grid barrier between sweeps (epochs would need 24 pollers per block)
+    // too many rounds for the caches: neighbours resolved every sweep
     for (int it = 0; it < sweeps; it++) {
       const float *src = (it & 1) ? D.pt : D.p;
       float *dst = (it & 1) ? D.p : D.pt;
       for (long long lc = first; lc < ncell; lc += stride)
         dst[base + lc] = jacobi_update(src, jacobi_neighbours(D, base + lc), alpha * D.div[base + lc]);
-      if (it + 1 < sweeps) barrier();
+      if (it + 1 < sweeps) bar.sync();
     }
   }
 }
@@ -526,7 +461,7 @@ int level_solve_grid(int sms) {
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_level_solve<0>, 256, 0) != cudaSuccess) return 0;
   return (a < b ? a : b) * sms;
 }
-void launch_level_solve(const Dev &D, int level, int prolong, int sweeps, int grid, int epoch_sync, cudaStream_t st) {
+void launch_level_solve(const Dev &D, int level, int prolong, int sweeps, int grid, cudaStream_t st) {
   // cells of the level are known only on the device; the cached variant
   // falls back to per-sweep neighbour resolution when they exceed its rounds,
   // and the uncached variant serves budgets that cannot fit at all.
@@ -542,8 +477,8 @@ void launch_level_solve(const Dev &D, int level, int prolong, int sweeps, int gr
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (cached) cudaLaunchKernelEx(&cfg, k_level_solve<LS_CACHE>, D, level, prolong, sweeps, epoch_sync);
-  else cudaLaunchKernelEx(&cfg, k_level_solve<0>, D, level, prolong, sweeps, epoch_sync == 2 ? 2 : 0);
+  if (cached) cudaLaunchKernelEx(&cfg, k_level_solve<LS_CACHE>, D, level, prolong, sweeps);
+  else cudaLaunchKernelEx(&cfg, k_level_solve<0>, D, level, prolong, sweeps);
 }
 
 // ------------------------------------------------------------------ batched kernels
@@ -793,7 +728,7 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
 template <int CACHE, int NB, int CLAIM>
 __device__ __forceinline__ void solve_pipelined(const SolveBatch &P, const long long *s_end, const int *s_lev,
                                                 uint32_t *s_cache, long long total, unsigned nctas, int sweeps,
-                                                int tree) {
+                                                GridBarrier &bar) {
   constexpr int W = 8, SX = DCG_TILE_SX, SY = DCG_TILE_SY, TILE = 5 * SX + 5 * SY + 8;
   __shared__ __align__(16) float s_pt[W][NB][TILE];
   __shared__ __align__(16) float s_pd[W][NB][64];
@@ -829,10 +764,6 @@ __device__ __forceinline__ void solve_pipelined(const SolveBatch &P, const long 
     const long long left = nblocks - g0;
     kcount += left <= 0 ? 0 : (left >= W ? W : (int)left);
   }
-  auto barrier = [&]() {
-    if (tree & 1) grid_barrier_tree(P.bar, P.err, nctas);
-    else grid_barrier(P.bar, P.err, nctas);
-  };
   // per buffer: arena index of the block's first cell and alpha (bits); own = ~0u: no block
   uint32_t b_own[NB], b_alpha[NB];
   // shared-memory addresses of the lane's copy targets in buffer 0 (buffer b: + b * TILE * 4)
@@ -961,7 +892,7 @@ __device__ __forceinline__ void solve_pipelined(const SolveBatch &P, const long 
       __syncwarp();  // buffer `buf` may be refilled by the next issue
     }
     cp_async_wait<0>();
-    if (it + 1 < sweeps) barrier();
+    if (it + 1 < sweeps) bar.sync();
   }
 }
 
@@ -969,7 +900,7 @@ __device__ __forceinline__ void solve_pipelined(const SolveBatch &P, const long 
 // one and whose level the cluster solve leaves (more than P.cl_max[m] blocks),
 // optional prolongation from the member's parent level, then `sweeps` Jacobi
 // sweeps over the concatenated cells of all members, separated by grid
-// barriers (tree & 1: two-level barrier). Member m's cells of the level
+// barriers. Member m's cells of the level
 // occupy [s_end[m-1], s_end[m]) of the concatenated index. With CACHE > 0 and
 // at most CACHE cells per thread, each thread keeps, per cell, the six
 // neighbour cells and its own cell as arena indices plus alpha*div in dynamic
@@ -979,7 +910,7 @@ __device__ __forceinline__ void solve_pipelined(const SolveBatch &P, const long 
 // of k_jacobi (identical results).
 template <int CACHE, int NB = 0, int MB = DCG_PIPE_MINB, int CLAIM = DCG_PIPE_CLAIM>
 __global__ void __launch_bounds__(256, NB ? MB : DCG_SOLVE_MINB)
-    k_level_solve_batch(const __grid_constant__ SolveBatch P, int sweeps, int tree) {
+    k_level_solve_batch(const __grid_constant__ SolveBatch P, int sweeps) {
   __shared__ long long s_end[BMAX];
   __shared__ int s_lev[BMAX];
   extern __shared__ __align__(16) uint32_t s_cache[];
@@ -1014,11 +945,8 @@ __global__ void __launch_bounds__(256, NB ? MB : DCG_SOLVE_MINB)
       if (s_lev[m] < P.d[m].g.levels - 1) prolong_cell(P.d[m], cell);
     }
   if (sweeps <= 0) return;
-  auto barrier = [&]() {
-    if (tree & 1) grid_barrier_tree(P.bar, P.err, nctas);
-    else grid_barrier(P.bar, P.err, nctas);
-  };
-  barrier();
+  GridBarrier bar(P.bar, P.err, nctas);
+  bar.sync();
   const int rounds = (int)((total + stride - 1) / stride);
   if (CACHE > 0 && rounds <= CACHE) {
     for (int r = 0; r < rounds; r++) {
@@ -1048,10 +976,10 @@ __global__ void __launch_bounds__(256, NB ? MB : DCG_SOLVE_MINB)
           dst[e[1536]] = jacobi_update(src, n, __uint_as_float(e[1792]));
         }
       }
-      if (it + 1 < sweeps) barrier();
+      if (it + 1 < sweeps) bar.sync();
     }
   } else if constexpr (NB > 0) {
-    solve_pipelined<CACHE, NB, CLAIM>(P, s_end, s_lev, s_cache, total, nctas, sweeps, tree);
+    solve_pipelined<CACHE, NB, CLAIM>(P, s_end, s_lev, s_cache, total, nctas, sweeps, bar);
   } else {
     // staged sweeps, one warp per block: per round each of the CTA's 8 warps
     // takes one block; its 64 cells and 96 face-halo cells go into a 6^3 tile
@@ -1178,7 +1106,7 @@ __global__ void __launch_bounds__(256, NB ? MB : DCG_SOLVE_MINB)
         __syncwarp();
         if (DCG_SOLVE_PIPE) cur = nxt;
       }
-      if (it + 1 < sweeps) barrier();
+      if (it + 1 < sweeps) bar.sync();
     }
   }
 }
@@ -1809,8 +1737,9 @@ void launch_check_div6(unsigned long long *bad, int sms, cudaStream_t st) {
 __global__ void __launch_bounds__(64) k_barrier_probe(uint32_t *bar, uint32_t *errw, unsigned limit,
                                                       unsigned absent) {
   if (blockIdx.x == absent) return;
-  grid_barrier(bar, errw, gridDim.x, limit);
-  grid_barrier(bar, errw, gridDim.x, limit);
+  GridBarrier b(bar, errw, gridDim.x);
+  b.sync(limit);
+  b.sync(limit);
 }
 int launch_barrier_probe(uint32_t *bar, uint32_t *errw, unsigned limit, unsigned nctas, cudaStream_t st) {
   unsigned absent = nctas - 1;
@@ -1931,7 +1860,7 @@ int batch_solve_grid(int sms, int cache, int ctas_per_sm) {
   const int k = (ctas_per_sm > 0 && ctas_per_sm < occ) ? ctas_per_sm : occ;
   return k * sms;
 }
-void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cache, int tree, cudaStream_t st) {
+void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cache, cudaStream_t st) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(256);
@@ -1944,19 +1873,19 @@ void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cac
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   switch (cache) {
-    case 8: cudaLaunchKernelEx(&cfg, k_level_solve_batch<8, 0>, P, sweeps, tree); break;
-    case 4: cudaLaunchKernelEx(&cfg, k_level_solve_batch<4, 0>, P, sweeps, tree); break;
-    case 3: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 0>, P, sweeps, tree); break;
-    case 16: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 2>, P, sweeps, tree); break;
-    case 32: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 3>, P, sweeps, tree); break;
-    case 18: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 2>, P, sweeps, tree); break;
-    case 19: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 2>, P, sweeps, tree); break;
-    case 34: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 3>, P, sweeps, tree); break;
-    case 35: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 3>, P, sweeps, tree); break;
-    case 64: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 2, 5>, P, sweeps, tree); break;
-    case 66: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 2, 5>, P, sweeps, tree); break;
-    case 83: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 2, 4, 1>, P, sweeps, tree); break;
-    default: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 0>, P, sweeps, tree); break;
+    case 8: cudaLaunchKernelEx(&cfg, k_level_solve_batch<8, 0>, P, sweeps); break;
+    case 4: cudaLaunchKernelEx(&cfg, k_level_solve_batch<4, 0>, P, sweeps); break;
+    case 3: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 0>, P, sweeps); break;
+    case 16: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 2>, P, sweeps); break;
+    case 32: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 3>, P, sweeps); break;
+    case 18: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 2>, P, sweeps); break;
+    case 19: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 2>, P, sweeps); break;
+    case 34: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 3>, P, sweeps); break;
+    case 35: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 3>, P, sweeps); break;
+    case 64: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 2, 5>, P, sweeps); break;
+    case 66: cudaLaunchKernelEx(&cfg, k_level_solve_batch<2, 2, 5>, P, sweeps); break;
+    case 83: cudaLaunchKernelEx(&cfg, k_level_solve_batch<3, 2, 4, 1>, P, sweeps); break;
+    default: cudaLaunchKernelEx(&cfg, k_level_solve_batch<0, 0>, P, sweeps); break;
   }
 }
 

@@ -354,14 +354,13 @@ typedef struct {
                                 64 + c (c = 0, 2): two, registers for 5 CTAs per SM;
                                 83: two, registers for 4 CTAs per SM, one block per claim */
   int32_t solve_ctas_per_sm; /* CTAs per SM of the cooperative solve (0 = occupancy limit) */
-  int32_t solve_barrier;     /* bit 0: grid barrier between sweeps, 0 flat, 1 two-level;
-                                bits 1 and 2 are accepted and without effect (every level
-                                goes to the solver that suits it, coarse to fine)        */
+  int32_t solve_barrier;     /* 0..7, accepted and without effect: one grid barrier between
+                                sweeps, every level to the solver that suits it           */
   int32_t persistent;        /* cell stages as persistent kernels over the allocated blocks */
   /* the solve_* fields schedule the grid-wide cooperative solve, which takes
    * the levels that the on-chip solves leave; for its round r < 4, its own
    * schedule when round_ctas_per_sm[r] != 0 (CTAs per SM, or -k: one CTA per k
-   * SMs; cache depth; barrier), else the solve_* fields above */
+   * SMs; cache depth; barrier without effect), else the solve_* fields above */
   int16_t round_ctas_per_sm[4];
   int8_t round_cache[4];
   int8_t round_barrier[4];

@@ -78,11 +78,12 @@ def test_subnormal_pressures_bitexact(scale):
     same(g, o)
 
 
-# dense levels of the adaptive grid: 16384 blocks (the smallest that takes the
-# dense passes) and an uneven box, with one, two and more passes of four sweeps
-# and a last one of two
+# full levels of the adaptive grid on both sides of the 36864 blocks that take
+# the dense passes (the first there has exactly as many), and uneven boxes, with
+# one, two and more passes of four sweeps and a last one of two
 @pytest.mark.parametrize("size,iters", [((256, 256, 128), 2), ((256, 256, 128), 4), ((128, 192, 360), 14),
-                                        ((1032, 64, 136), 6)])
+                                        ((1032, 64, 136), 6), ((256, 256, 288), 2), ((256, 256, 288), 4),
+                                        ((384, 120, 440), 14), ((2064, 64, 144), 6)])
 def test_dense_level_bitexact(size, iters):
     gx, gy, gz = size
     full1 = (gx // 8) * (gy // 8) * (gz // 8)
