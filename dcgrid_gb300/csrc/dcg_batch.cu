@@ -233,7 +233,7 @@ struct dcg_batch {
           P.lev[i] = lev[g + i];
           P.cl_max[i] = limit;
         }
-        launch_level_solve_batch(P, iters, grid, cache, stream);
+        if (!launch_resident_solve(P, iters, sms, stream)) launch_level_solve_batch(P, iters, grid, cache, stream);
       }
     });
   }

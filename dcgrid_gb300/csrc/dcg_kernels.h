@@ -121,6 +121,12 @@ int batch_solve_grid(int sms, int cache, int ctas_per_sm);
 bool solve_variant_valid(int cache);
 void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cache, cudaStream_t st);
 
+// k_resident.cu: the same solve, and a level's sweeps transposed, with the
+// cells in registers; false: too many blocks (or a form that they do not take)
+bool launch_resident_solve(const SolveBatch &P, int sweeps, int sms, cudaStream_t st);
+bool launch_resident_adjoint(const Dev &D, int level, int sweeps, float *lp0, float *lp1, float *ld, int sms,
+                             cudaStream_t st);
+
 // k_cascade.cu: cluster size of the device's cluster solve (0: none), blocks a
 // cluster of that size holds, and the launch (it picks P.csize)
 int cluster_solve_size();
@@ -176,9 +182,10 @@ struct Cascade {
   int sms = 148;
   int sweeps = 0, prolong = 1;
   cudaStream_t st = nullptr;
-  // blocks that make the dense solve the faster one (a box of 32768 blocks: 8.3
-  // us per sweep, grid-wide 7.7; of 65536: 8.5 and 13.0)
-  static constexpr long long kDenseBlocks = 36864;
+  // blocks that make the dense solve the faster one: more than the resident
+  // solve holds on 152 SMs (us per sweep of 36864 blocks: dense 11.4, resident
+  // 6.2; of 65536: dense 8.5, k_level_solve_batch 13.0)
+  static constexpr long long kDenseBlocks = 38913;
   long long limit() const { return csize > 0 ? cluster_solve_blocks(csize) : 0; }
   // general(members, levels, limit, round): solve levels[i] of members[i]
   // unless at most `limit` of its blocks are allocated

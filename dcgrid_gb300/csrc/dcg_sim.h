@@ -648,7 +648,8 @@ struct dcg_sim {
     SB.lev[0] = level;
     SB.cl_max[0] = limit;
     SB.d[0] = d;
-    launch_level_solve_batch(SB, sweeps, ls_grid_staged, kSolveVariant, stream);
+    if (!launch_resident_solve(SB, sweeps, sms, stream))
+      launch_level_solve_batch(SB, sweeps, ls_grid_staged, kSolveVariant, stream);
   }
   void a_advect_scalars() {
     cells(1, 1);

@@ -465,7 +465,8 @@ void launch_adjoint_full_phase_a(const Dev &DA, const AdjFull &A, float *lam_em,
   const int top = DA.g.levels - 1;
   for (int level = 0; level <= top; level++) {
     const unsigned g = adj_grid(DA.g.budget[level]);
-    for (int it = sweeps - 1; it >= 0; it--) {
+    const bool done = launch_resident_adjoint(DA, level, sweeps, A.lp0, A.lp1, A.ld, sms, st);
+    for (int it = sweeps - 1; !done && it >= 0; it--) {
       // sweep it read src = (it odd ? p~ : p) and wrote dst = the other plane
       float *ldst = (it & 1) ? A.lp0 : A.lp1, *lsrc = (it & 1) ? A.lp1 : A.lp0;
       k_adj_jacobi<<<g, 256, 0, st>>>(DA, level, ldst, lsrc, A.ld);

@@ -78,12 +78,13 @@ def test_subnormal_pressures_bitexact(scale):
     same(g, o)
 
 
-# full levels of the adaptive grid on both sides of the 36864 blocks that take
-# the dense passes (the first there has exactly as many), and uneven boxes, with
+# full levels of the adaptive grid on both sides of the 38912 blocks that the
+# resident solve holds, beyond which dense passes take them, and uneven boxes, with
 # one, two and more passes of four sweeps and a last one of two
 @pytest.mark.parametrize("size,iters", [((256, 256, 128), 2), ((256, 256, 128), 4), ((128, 192, 360), 14),
-                                        ((1032, 64, 136), 6), ((256, 256, 288), 2), ((256, 256, 288), 4),
-                                        ((384, 120, 440), 14), ((2064, 64, 144), 6)])
+                                        ((1032, 64, 136), 6), ((256, 256, 304), 2), ((256, 256, 312), 2),
+                                        ((256, 256, 312), 4),
+                                        ((384, 120, 440), 14), ((2064, 64, 152), 6)])
 def test_dense_level_bitexact(size, iters):
     gx, gy, gz = size
     full1 = (gx // 8) * (gy // 8) * (gz // 8)
@@ -159,3 +160,60 @@ def test_many_moves_and_refinements(blocks, compat):
             assert np.array_equal(tg[k], to[k])
         most = max(most, len(mo))
     print("largest number of moves:", most)
+
+
+# Levels too large for a cluster: budgets of one, two, four and eight block
+# pairs per warp and beyond what the chip holds (38912 blocks), odd counts,
+# with coarser neighbours, domain faces and the compat quirk
+@pytest.mark.parametrize("compat", [0, 1])
+@pytest.mark.parametrize("size,blocks,iters", [((128, 64, 64), 3001, 6), ((64, 128, 128), 6553, 4),
+                                               ((128, 128, 128), 18999, 4), ((128, 136, 128), 21111, 2), ((128, 192, 128), 40001, 2)])
+def test_resident_levels_bitexact(size, blocks, iters, compat):
+    gx, gy, gz = size
+    full1 = (gx // 8) * (gy // 8) * (gz // 8)
+    p = scenarios.plume(gx, gy, gz, full1 + blocks, 2, iters)
+    p.src_radius = min(size) / 4.0
+    p.ref_compat = compat
+    g, o = pair(p, 0.5)
+    for s in (g, o):
+        s.step(2)
+        s.project_local()
+    g.sync()
+    assert g.get_topology()["load"][0] > 2048
+    same(g, o)
+
+
+# The transposed projection alone: in a flow at rest the advections' transposes
+# are the identity in FP32 and FP64, so a random velocity adjoint meets only the
+# pressure path. Bound: 20 sweeps and the prolongation of about 10 roundings
+# each in FP32, 1.2e-5, times 8 for the sums they end in.
+@pytest.mark.parametrize("g,blocks,iters,compat", [(64, 3600, 20, 0), (96, 5529, 6, 0), (96, 12441, 20, 0),
+                                                   (96, 5529, 6, 1), (112, 20001, 4, 0), (32, 100, 2, 0)])
+def test_transposed_projection_matches_fp64(g, blocks, iters, compat):
+    import torch
+    from dcgrid_gb300 import Simulation
+    from oracle.pyoracle import OracleSim
+    p = scenarios.differentiable(g, 2, iters=iters)
+    p.max_blocks = (g // 8) ** 3 + blocks
+    p.ref_compat = compat
+    s = Simulation(p)
+    s.step(2)
+    s.sync()
+    o = OracleSim(p, precision="double")
+    o.set_topology(s.get_topology())
+    for f in ["density", "fluidity", "vel_x", "vel_y", "vel_z"]:
+        o.set_field(f, s.get_field(f).astype(np.float64))
+    nc = 64 * p.max_blocks
+    alloc = np.repeat(o.get_topology()["pos"][:, 3] >= 0, 64)
+    lam = np.zeros(4 * nc, np.float32)
+    lam[:3 * nc] = np.random.default_rng(11).standard_normal(3 * nc) * np.tile(alloc, 3)
+    li = torch.from_numpy(lam).cuda()
+    lo = torch.empty_like(li)
+    s.adjoint_step_full(li, lo)
+    torch.cuda.synchronize()
+    mv, rf = s.get_last_adapt()
+    want = o.adjoint_step_full(lam.astype(np.float64), moves=mv, refines=rf)
+    got = lo.cpu().numpy().astype(np.float64)
+    for d in range(3):
+        a, b = got[d * nc:(d + 1) * nc], want[d * nc:(d + 1) * nc]
+        assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b)
