@@ -639,8 +639,16 @@ int dcg_render(dcg_sim *s, const dcg_render_params *rp, float *rgba, int32_t whe
     }
     out = reinterpret_cast<float4 *>(s->render_tmp);
   }
-  if (s->mode == DCG_MODE_ADAPTIVE) launch_render_adaptive(s->D, R, out, s->stream);
-  else launch_render_uniform(s->U, R, out, s->stream);
+  if (s->mode == DCG_MODE_ADAPTIVE) {
+    // the frame's scratch is kept for the next one: its size is the handle's
+    const size_t need = render_scratch_bytes(s->D.g, R);
+    if (need && !s->render_scratch && cudaMalloc(&s->render_scratch, need) != cudaSuccess) {
+      cudaGetLastError();
+      s->render_scratch = nullptr;
+    }
+    if (need && s->render_scratch) launch_render_tiled(s->D, R, s->render_scratch, out, s->stream);
+    else launch_render_adaptive(s->D, R, out, s->stream);
+  } else launch_render_uniform(s->U, R, out, s->stream);
   if ((rc = s->check_launch("render"))) return rc;
   if (where != DCG_DEVICE &&
       (rc = s->cuda(cudaMemcpyAsync(rgba, out, n * 16, cudaMemcpyDeviceToHost, s->stream), "render")))

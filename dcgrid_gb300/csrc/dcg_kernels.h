@@ -262,6 +262,9 @@ void launch_u_advect_scalars(const UDev &U, bool apply, cudaStream_t st);  // ap
 void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, bool apply, int sms, cudaStream_t st);
 void launch_u_add_noise(const UDev &U, unsigned long long seed, float amp, cudaStream_t st);
 void launch_u_stats(const UDev &U, cudaStream_t st);
+// bytes of a frame's scratch (0: the frame takes launch_render_adaptive)
+size_t render_scratch_bytes(const Geom &g, const RenderP &R);
+void launch_render_tiled(const Dev &D, const RenderP &R, void *scratch, float4 *out, cudaStream_t st);
 void launch_render_adaptive(const Dev &D, const RenderP &R, float4 *out, cudaStream_t st);
 void launch_render_uniform(const UDev &U, const RenderP &R, float4 *out, cudaStream_t st);
 

@@ -126,6 +126,7 @@ struct dcg_sim {
   uint32_t *afull_parent = nullptr, *afull_child = nullptr, *afull_nbr = nullptr;
   float *render_tmp = nullptr; // renderer output staging for host buffers
   size_t render_cap = 0;
+  void *render_scratch = nullptr;  // density tiles and leaf map of the frame (allocated on first use)
   float *hmap = nullptr;       // terrain heightmap (dcg_set_heightmap), or null
   int hm_nx = 0, hm_nz = 0;
   int vpar = 0, qpar = 0;
@@ -201,6 +202,7 @@ struct dcg_sim {
   }
   ~dcg_sim() {
     if (render_tmp) cudaFree(render_tmp);
+    if (render_scratch) cudaFree(render_scratch);
     if (hmap) cudaFree(hmap);
     free_all();
     if (own_stream && stream) cudaStreamDestroy(stream);

@@ -38,6 +38,11 @@ __device__ inline void mix(F3 src, float srcAlpha, F3 &dst, float &dstAlpha) {
   }
 }
 
+// A map word: leaf block, its level, whether its tile holds zeros only. A tile:
+// the block's cells and apron, [x][y][z].
+constexpr int RT_LEVEL = 24, RT_CELLS = 6 * 6 * 6;
+constexpr uint32_t RT_BLOCK = 0xFFFFFFu, RT_EMPTY = 0x80000000u;
+
 struct March {  // MarchAux (raymarching.cuh:19-43)
   int ix, iy, iz;
   float fx, fy, fz;
@@ -61,6 +66,8 @@ template <class Field> __device__ inline float interp(const March &a, Field f) {
 // Adaptive grid samplers (dcgrid_rendering.cu:6-56): the finest block over the
 // sample, then either its nearest cell or a trilinear read of its apron.
 struct AdaptiveGrid {
+  static constexpr int kAhead = 1;
+  static constexpr bool kSlices = true;
   const Dev &D;
   __device__ float q(size_t i) const { return q_ld(D, 0, i); }
   __device__ const Geom &g() const { return D.g; }
@@ -112,8 +119,107 @@ struct AdaptiveGrid {
   }
 };
 
+// The adaptive grid's precise or nearest density through the scratch that a
+// frame fills first (k_render_tiles, k_render_map): the sample's leaf block from
+// a map over the finest blocks, its eight corners from the block's own copy of
+// its cells and apron. That is two dependent loads; walking the tree and
+// resolving eight apron cells through the neighbour table were five or six.
+// Blocks whose copy holds zeros only need the map alone. The results are
+// AdaptiveGrid's.
+struct TiledGrid {
+  static constexpr int kAhead = 4;
+  static constexpr bool kSlices = false;
+  const Dev &D;
+  const float *tile;
+  const uint32_t *map;
+  __device__ const Geom &g() const { return D.g; }
+  __device__ const Phys &ph() const { return D.ph; }
+  __device__ __forceinline__ uint32_t leaf(F3 p, int &ix, int &iy, int &iz) const {
+    ix = clampi((int)floorf(p.x), 0, D.g.gx - 1);
+    iy = clampi((int)floorf(p.y), 0, D.g.gy - 1);
+    iz = clampi((int)floorf(p.z), 0, D.g.gz - 1);
+    return __ldg(map + ((ix >> 2) * (D.g.gy >> 2) + (iy >> 2)) * (D.g.gz >> 2) + (iz >> 2));
+  }
+  // the density at each of N positions, those with on[i] set
+  template <int N>
+  __device__ __forceinline__ void densities(const F3 (&p)[N], const bool (&on)[N], bool precise,
+                                            float (&out)[N]) const {
+    int ix[N], iy[N], iz[N];
+    uint32_t e[N];
+#pragma unroll
+    for (int n = 0; n < N; n++) e[n] = leaf(p[n], ix[n], iy[n], iz[n]);
+    float c[N][8], f[N][3];
+    bool far = false;  // a position outside its block's apron (it is not in the domain): the tree's answer
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      const int lev = (int)(e[n] >> RT_LEVEL) & 15;
+      const float *T = tile + (size_t)(e[n] & RT_BLOCK) * RT_CELLS;
+      const float sum = p[n].x + p[n].y + p[n].z;
+      const bool read = on[n] && !((e[n] & RT_EMPTY) && sum - sum == 0.f);
+      if (precise) {
+        const float si = __int_as_float((127 - lev) << 23);
+        const float x = p[n].x * si - .5f, y = p[n].y * si - .5f, z = p[n].z * si - .5f;
+        const float xf = floorf(x), yf = floorf(y), zf = floorf(z);
+        f[n][0] = x - xf;
+        f[n][1] = y - yf;
+        f[n][2] = z - zf;
+        const int i = (int)xf + 1 - ((ix[n] >> lev) & ~3), j = (int)yf + 1 - ((iy[n] >> lev) & ~3),
+                  k = (int)zf + 1 - ((iz[n] >> lev) & ~3);
+        const bool in = (unsigned)i <= 4u && (unsigned)j <= 4u && (unsigned)k <= 4u;
+        far = far || (read && !in);
+        T += (i * 6 + j) * 6 + k;
+        c[n][0] = c[n][1] = c[n][2] = c[n][3] = c[n][4] = c[n][5] = c[n][6] = c[n][7] = 0.f;
+        if (read && in) {
+          c[n][0] = T[0];
+          c[n][1] = T[1];
+          c[n][2] = T[6];
+          c[n][3] = T[7];
+          c[n][4] = T[36];
+          c[n][5] = T[37];
+          c[n][6] = T[42];
+          c[n][7] = T[43];
+        }
+      } else {
+        const int sh = D.g.ref_compat ? 0 : lev;
+        T += ((((ix[n] >> sh) & 3) + 1) * 6 + ((iy[n] >> sh) & 3) + 1) * 6 + ((iz[n] >> sh) & 3) + 1;
+        out[n] = read ? T[0] : 0.f;
+      }
+    }
+    if (!precise) return;
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      March a;
+      a.fx = f[n][0];
+      a.fy = f[n][1];
+      a.fz = f[n][2];
+#pragma unroll
+      for (int q = 0; q < 8; q++) a.idx[q] = q;
+      out[n] = interp(a, [&](size_t q) { return c[n][q]; });
+    }
+    if (far) {
+#pragma unroll
+      for (int n = 0; n < N; n++)
+        if (on[n]) out[n] = by_tree(p[n]);
+    }
+  }
+  __device__ __noinline__ float by_tree(F3 p) const {
+    March a;
+    AdaptiveGrid{D}.sample(p, true, a);
+    return a.density;
+  }
+  __device__ __forceinline__ void sample(F3 p, bool precise, March &a) const {
+    const F3 pp[1] = {p};
+    const bool on[1] = {true};
+    float d[1];
+    densities(pp, on, precise, d);
+    a.density = d[0];
+  }
+};
+
 // Uniform grid samplers (uniformgrid_rendering.cu:5-52)
 struct UniformGridR {
+  static constexpr int kAhead = 1;
+  static constexpr bool kSlices = true;
   const UDev &U;
   __device__ const Geom &g() const { return U.g; }
   __device__ const Phys &ph() const { return U.ph; }
@@ -207,11 +313,30 @@ __device__ float light_march(const Grid &G, const RenderP &R, F3 origin, F3 sun,
       }
       const float step = fmaxf(dFar / 100.f, 1e-1f);
       float dens = 0.f;
-      March a;
-      for (float d = step; d < dFar && dens < 5.f; d += step) {
-        pos = pos + sun * step;
-        G.sample(pos, R.precise != 0, a);
-        dens += a.density * ph.dx * step;
+      if constexpr (Grid::kAhead > 1) {  // samples fetched ahead, added in order up to the one that ends the march
+        float d = step;
+        while (d < dFar && dens < 5.f) {
+          F3 p[Grid::kAhead];
+          bool on[Grid::kAhead];
+          float v[Grid::kAhead];
+#pragma unroll
+          for (int n = 0; n < Grid::kAhead; n++) {
+            p[n] = pos = pos + sun * step;
+            on[n] = d < dFar;
+            d += step;
+          }
+          G.densities(p, on, R.precise != 0, v);
+#pragma unroll
+          for (int n = 0; n < Grid::kAhead; n++)
+            if (on[n] && dens < 5.f) dens += v[n] * ph.dx * step;
+        }
+      } else {
+        March a;
+        for (float d = step; d < dFar && dens < 5.f; d += step) {
+          pos = pos + sun * step;
+          G.sample(pos, R.precise != 0, a);
+          dens += a.density * ph.dx * step;
+        }
       }
       light *= expf(-dens);
     }
@@ -284,21 +409,22 @@ __device__ float4 ray_march(const Grid &G, const RenderP &R, F3 origin, F3 dir, 
   }
   F3 pos = origin + dir * dSolid;
   const float bgAlpha = density_alpha(ph.dx, dSolid, 1e-6f);
+  if (what == 2) pos.y = 0.f;
+  float shade = 1.f;
+  if (R.shadows && (what == 1 || what == 2)) shade = light_march(G, R, pos, sun, suninv);
   if (what == 1) {
     light = fmaxf(0.f, dot3(sdf_normal(g, ph, pos), sun));
-    if (R.shadows) light *= light_march(G, R, pos, sun, suninv);
+    light *= shade;
     light = R.ambient + light * ambInv;
     mix(f3(R.scene[0], R.scene[1], R.scene[2]) * light, 1.f - bgAlpha, color, alpha);
   }
   if (what == 2) {
-    pos.y = 0.f;
-    light = floorLight;
-    if (R.shadows) light *= light_march(G, R, pos, sun, suninv);
+    light = floorLight * shade;
     light = R.ambient + light * ambInv;
     light *= 1.f + .1f * fmodf(fabsf(floorf(pos.x / g.gx) + floorf(pos.z / g.gx)), 2.f);
     mix(f3(R.floor_[0], R.floor_[1], R.floor_[2]) * light, 1.f - bgAlpha, color, alpha);
   }
-  if (what == 3) {
+  if constexpr (Grid::kSlices) if (what == 3) {
     pos.z = sliceZ;
     G.sample(pos, R.precise != 0, a);
     if (R.channel == CH_DENSITY) mix(f3(a.density * 1e2f, 0.f, 0.f), 1.f, color, alpha);
@@ -337,6 +463,45 @@ template <class Grid> __device__ float4 render_pixel(const Grid &G, const Render
   return make_float4(acc.x * n, acc.y * n, acc.z * n, acc.w * n);
 }
 
+// one warp per block: its tile, and whether that holds anything
+__global__ void __launch_bounds__(256) k_render_tiles(const __grid_constant__ Dev D, float *tile, uint8_t *empty) {
+  const long long b = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (b >= D.g.B) return;
+  const int4 bp = D.pos[b];
+  if (bp.w < 0) return;
+  float *T = tile + (size_t)b * RT_CELLS;
+  bool any = false;
+  for (int c = threadIdx.x & 31; c < RT_CELLS; c += 32) {
+    const float v = q_ld(D, 0, apron_cell(D, (uint32_t)b, bp, c / 36, c / 6 % 6, c % 6));
+    T[c] = v;
+    any |= v != 0.f;
+  }
+  any = __any_sync(0xffffffffu, any);
+  if ((threadIdx.x & 31) == 0) empty[b] = !any;
+}
+// one thread per finest block: the leaf over it
+__global__ void __launch_bounds__(256) k_render_map(const __grid_constant__ Dev D, const uint8_t *empty,
+                                                    uint32_t *map) {
+  const int ny = D.g.gy >> 2, nz = D.g.gz >> 2, n = (D.g.gx >> 2) * ny * nz;
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  int lev;
+  const uint32_t b = locate(D, 4 * (i / (ny * nz)), 4 * (i / nz % ny), 4 * (i % nz), 0, lev);
+  map[i] = b | (uint32_t)lev << RT_LEVEL | (empty[b] ? RT_EMPTY : 0u);
+}
+// 8 by 8 pixels per CTA, 8 by 4 per warp: rays of a warp meet the same blocks
+// and smoke, and small CTAs even out the rays' lengths. What bounds it is the
+// chain of dependent loads along a ray, up to a hundred sun samples for each of
+// its own: four samples in flight and registers for all of them (640 x 360
+// over 64 x 128 x 64 cells with shadows, us: walking the tree 8200; 1, 2, 4, 8
+// ahead at 8 CTAs per SM 1259, 1101, 1076, -; 4 ahead at 6, 4, 2 CTAs 1087,
+// 932, 964; 8 ahead at 4 and 2 1158, 1140).
+__global__ void __launch_bounds__(64, 4) k_render_tiled(const __grid_constant__ Dev D, const __grid_constant__ RenderP R,
+                                                     const float *tile, const uint32_t *map, float4 *out) {
+  const int x = blockIdx.x * 8 + (threadIdx.x & 7), y = blockIdx.y * 8 + (threadIdx.x >> 3);
+  if (x >= R.width || y >= R.height) return;
+  out[(size_t)y * R.width + x] = render_pixel(TiledGrid{D, tile, map}, R, x, y);
+}
 __global__ void __launch_bounds__(256) k_render_adaptive(const __grid_constant__ Dev D, const __grid_constant__ RenderP R,
                                                          float4 *out) {
   const int x = blockIdx.x * 16 + (threadIdx.x & 15), y = blockIdx.y * 16 + (threadIdx.x >> 4);
@@ -352,6 +517,25 @@ __global__ void __launch_bounds__(256) k_render_uniform(const __grid_constant__ 
 
 }  // namespace
 
+// The scratch is 865 bytes per block and four per finest block: past 2^18
+// blocks (228 MB) frames walk the tree instead. It takes two launches of some
+// 5 us to fill for 5120 blocks; the debug slices read a sample per pixel and
+// have no use for it.
+size_t render_scratch_bytes(const Geom &g, const RenderP &R) {
+  const long long n = (long long)(g.gx >> 2) * (g.gy >> 2) * (g.gz >> 2);
+  if (R.channel != CH_FLUID || g.B > (1 << 18) || n > (1 << 24)) return 0;
+  return (size_t)g.B * (RT_CELLS * 4 + 1) + (size_t)n * 4;
+}
+void launch_render_tiled(const Dev &D, const RenderP &R, void *scratch, float4 *out, cudaStream_t st) {
+  float *tile = reinterpret_cast<float *>(scratch);
+  uint32_t *map = reinterpret_cast<uint32_t *>(tile + (size_t)D.g.B * RT_CELLS);
+  const int n = (D.g.gx >> 2) * (D.g.gy >> 2) * (D.g.gz >> 2);
+  uint8_t *empty = reinterpret_cast<uint8_t *>(map + n);
+  k_render_tiles<<<(unsigned)((D.g.B + 7) / 8), 256, 0, st>>>(D, tile, empty);
+  k_render_map<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(D, empty, map);
+  const dim3 grid((unsigned)((R.width + 7) / 8), (unsigned)((R.height + 7) / 8));
+  k_render_tiled<<<grid, 64, 0, st>>>(D, R, tile, map, out);
+}
 void launch_render_adaptive(const Dev &D, const RenderP &R, float4 *out, cudaStream_t st) {
   const dim3 grid((unsigned)((R.width + 15) / 16), (unsigned)((R.height + 15) / 16));
   k_render_adaptive<<<grid, 256, 0, st>>>(D, R, out);

@@ -75,3 +75,30 @@ def test_render_into_device_memory():
     host = g.render(rp)
     dev = g.render(rp, torch.empty((rp.height, rp.width, 4), dtype=torch.float32, device="cuda"))
     assert np.array_equal(dev.cpu().numpy(), host)
+
+
+@pytest.mark.parametrize("precision", [capi.PRECISION_FP32, capi.PRECISION_MIXED_FP16, capi.PRECISION_MIXED])
+@pytest.mark.parametrize("precise,compat", [(1, 0), (1, 1), (0, 0)])
+def test_sparse_levels_inside_the_domain_and_frame_after_frame(precision, precise, compat):
+    """Leaves of three levels, an eye inside the grid, image sides that are no
+    multiple of a tile, and a second frame after the state has changed. The
+    smoke is made dense: an alpha near 1e-6 is the difference of 1 and an
+    exponential, where the two libraries' roundings would show in the colour."""
+    p = scenarios.plume(48, 64, 80, 120 + 300, 3, 6)
+    p.precision, p.ref_compat = precision, compat
+    p.refine_criterion = capi.REFINE_GEOMETRIC
+    g, o = gpu(p), orc(p, "float")
+    g.add_velocity_noise(1, 2.0)
+    rp = render_params(p, 37, 23, shadows=1, precise=precise)
+    for steps in (4, 3):
+        g.step(steps)
+        g.sync()
+        smoke = g.get_field("density")
+        g.set_field("density", np.where(smoke > 0.05, smoke + 0.2, 0.0).astype(np.float32))
+        o.set_topology(g.get_topology())
+        for f in ("density", "fluidity"):
+            o.set_field(f, g.get_field(f))
+        image = g.render(rp)
+        assert (image[..., 3] > 0.1).any()
+        close(image, o.render(rp), steps)
+        rp.eye[0], rp.eye[1], rp.eye[2] = 0.4 * p.gx * p.dx, 0.2 * p.gy * p.dx, 0.1 * p.gz * p.dx
