@@ -395,7 +395,12 @@ int cluster_solve_size() {
   }
   return 0;
 }
-long long cluster_solve_blocks(int csize) { return (long long)csize * CL_BLOCKS; }
+// The levels that go to a cluster: one group of blocks per warp. The second
+// group is for launches of many members, whose clusters are smaller: alone, a
+// level that needs it is faster with the whole GPU (us per sweep: 1830 sparse
+// blocks 3.3 here, 2.0 in the resident solve, 1728 full ones 2.0 and 1.85; of
+// 1024 full blocks 1.4 and 1.8).
+long long cluster_solve_blocks(int csize) { return (long long)csize * CL_WARPS * 4; }
 
 // max_blocks: the largest level of the launch. CTAs per cluster: about one
 // group of blocks per warp, but no more than the clusters of all members fit
