@@ -138,30 +138,32 @@ struct Halo {
 // The halo values of a quad as loaded: on a face to a coarser block the aligned
 // vector that holds the coarser cell (rs_fix picks it when the loads are due).
 // Loads go to L2: the planes are rewritten by other SMs within the launch.
-__device__ __forceinline__ void rs_load(const float *__restrict__ src, const Quad &q, const uint4 &r, int h, Halo &o) {
+__device__ __forceinline__ void rs_load(const float *__restrict__ src, const Quad &q, const uint4 &r, Halo &o) {
   o.x = make_float4(0.f, 0.f, 0.f, 0.f);
   if ((q.fl & (RS_X | RS_XQ)) == RS_X) o.x = __ldcg(reinterpret_cast<const float4 *>(src + (q.x & ~3u)));
   if (!(q.fl & RS_YQ)) o.y = __ldcg(reinterpret_cast<const float2 *>(src + (r.x & ~1u)));
   o.z0 = __ldcg(src + r.y);
   o.z1 = __ldcg(src + r.z);
-  if (!(q.fl & RS_QUIRK)) return;  // uniform in the warp
-  const int x = 2 * ((h >> 3) & 1) + (h & 1), y = 2 * ((h >> 2) & 1), z = 2 * ((h >> 1) & 1);
-  if (q.fl & RS_XQ) {
-    const float *s = src + q.x;
-    const int qx = x ? 0 : 1;
-    o.x.x = __ldcg(s + local_of(qx, (y + 1) & 3, (z + 1) & 3));
-    o.x.y = __ldcg(s + local_of(qx, (y + 1) & 3, (z + 2) & 3));
-    o.x.z = __ldcg(s + local_of(qx, (y + 2) & 3, (z + 1) & 3));
-    o.x.w = __ldcg(s + local_of(qx, (y + 2) & 3, (z + 2) & 3));
-  }
-  if (q.fl & RS_YQ) {
-    const int qy = y ? 0 : 1;
-    o.y.x = __ldcg(src + r.x + local_of((x + 1) & 3, qy, (z + 1) & 3));
-    o.y.y = __ldcg(src + r.x + local_of((x + 1) & 3, qy, (z + 2) & 3));
-  }
 }
-// ADJ: a coarser neighbour contributes nothing.
-template <bool ADJ> __device__ __forceinline__ void rs_fix(const Quad &q, const uint4 &r, Halo &o) {
+// ADJ: a coarser neighbour contributes nothing. The compat boundary's cells on
+// x and y faces are the block's own, shifted by one along every axis: they
+// come from the lanes that hold them (a second load into the same registers
+// would wait for the first: 1283 blocks 2.46 us per sweep, with shuffles 1.92).
+template <bool ADJ> __device__ __forceinline__ void rs_fix(const Quad &q, const uint4 &r, int h, Halo &o) {
+  if (q.fl & RS_QUIRK) {  // uniform in the warp
+    const unsigned all = 0xffffffffu;
+    const int top = threadIdx.x & 16, x1 = h & 8, y1 = h & 4, z1 = h & 2, x0 = h & 1;
+    // x face: (1 or 0, y + 1 or y + 2, z + 1 or z + 2), modulo 4
+    const int fx = top | (x0 ^ 1);
+    const float a = __shfl_sync(all, q.v[3], fx | y1 | z1), b = __shfl_sync(all, q.v[2], fx | y1 | (z1 ^ 2)),
+                c = __shfl_sync(all, q.v[1], fx | (y1 ^ 4) | z1), d = __shfl_sync(all, q.v[0], fx | (y1 ^ 4) | (z1 ^ 2));
+    // y face: (x + 1, 1 or 0, z + 1 or z + 2)
+    const int fy = top | (x0 ? x1 ^ 8 : x1) | (x0 ^ 1);
+    const float e0 = __shfl_sync(all, q.v[1], fy | z1), e1 = __shfl_sync(all, q.v[3], fy | z1),
+                f0 = __shfl_sync(all, q.v[0], fy | (z1 ^ 2)), f1 = __shfl_sync(all, q.v[2], fy | (z1 ^ 2));
+    if (q.fl & RS_XQ) o.x = make_float4(a, b, c, d);
+    if (q.fl & RS_YQ) o.y = make_float2(y1 ? e0 : e1, y1 ? f0 : f1);
+  }
   if (!(q.fl & RS_SLOW)) return;  // uniform in the warp
   if (q.fl & RS_XC) {
     const float a = q.x & 1u ? o.x.y : o.x.x, b = q.x & 1u ? o.x.w : o.x.z, c = ADJ ? 0.f : q.x & 2u ? b : a;
@@ -215,24 +217,11 @@ __device__ __forceinline__ void rs_flags(Quad &q) {
   if (__any_sync(0xffffffffu, q.fl & (RS_XQ | RS_YQ))) q.fl |= RS_QUIRK;
 }
 
+// s_end[m]: the blocks of members 0..m
 template <int K>
-__global__ void __launch_bounds__(RS_WARPS * 32, 1) k_resident_solve(const __grid_constant__ SolveBatch P, int sweeps) {
-  __shared__ long long s_end[BMAX];
+__device__ __forceinline__ void rs_solve(const SolveBatch &P, const long long *s_end, long long total, int sweeps,
+                                         GridBarrier &bar) {
   const int t = threadIdx.x, h = t & 15;
-  if (t == 0) {
-    long long acc = 0;
-    for (int m = 0; m < P.n; m++) {
-      if (P.lev[m] >= 0) {
-        const long long load = __ldcg(P.d[m].load + P.lev[m]);
-        if (load > P.cl_max[m]) acc += load;
-      }
-      s_end[m] = acc;
-    }
-  }
-  __syncthreads();
-  const long long total = s_end[P.n - 1];
-  if (total == 0) return;  // the cluster solve took every level: the same in every CTA
-  GridBarrier bar(P.bar, P.err, gridDim.x);
   const int warps = blockDim.x >> 5;
   Quad q[K];
   Rests<K> rest;
@@ -280,15 +269,15 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 1) k_resident_solve(const __gri
     const float *src = (it & 1) ? P.pt : P.p;
     float *dst = (it & 1) ? P.p : P.pt;
     Halo hv, next;  // two pairs' halos in flight: more do not fit the registers
-    rs_load(src, q[0], rest.at(0), h, hv);
+    rs_load(src, q[0], rest.at(0), hv);
 #pragma unroll
     for (int k = 0; k < K; k++) {
       if (k >= pairs) break;
-      if (k + 1 < K && k + 1 < pairs) rs_load(src, q[k + 1 < K ? k + 1 : k], rest.at(k + 1 < K ? k + 1 : k), h, next);
+      if (k + 1 < K && k + 1 < pairs) rs_load(src, q[k + 1 < K ? k + 1 : k], rest.at(k + 1 < K ? k + 1 : k), next);
       const uint4 r = rest.at(k);
       const float4 ad = rest.ad(k);
       float2 s[2];
-      rs_fix<false>(q[k], r, hv);
+      rs_fix<false>(q[k], r, h, hv);
       rs_sums(q[k], hv, h, s);
       s[0] = __fadd2_rn(s[0], make_float2(-ad.x, -ad.y));
       s[1] = __fadd2_rn(s[1], make_float2(-ad.z, -ad.w));
@@ -301,6 +290,32 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 1) k_resident_solve(const __gri
       hv = next;
     }
   }
+}
+
+// One kernel for every number of pairs per warp: the host knows the budgets
+// only, and a level far below its budget would pay for pairs that it has not
+// (6891 of 17952 blocks: 2.56 us per sweep with four pairs, 2.42 with two).
+__global__ void __launch_bounds__(RS_WARPS * 32, 1) k_resident_solve(const __grid_constant__ SolveBatch P, int sweeps) {
+  __shared__ long long s_end[BMAX];
+  if (threadIdx.x == 0) {
+    long long acc = 0;
+    for (int m = 0; m < P.n; m++) {
+      if (P.lev[m] >= 0) {
+        const long long load = __ldcg(P.d[m].load + P.lev[m]);
+        if (load > P.cl_max[m]) acc += load;
+      }
+      s_end[m] = acc;
+    }
+  }
+  __syncthreads();
+  const long long total = s_end[P.n - 1];
+  if (total == 0) return;  // the cluster solve took every level: the same in every CTA
+  GridBarrier bar(P.bar, P.err, gridDim.x);
+  const long long one = (long long)gridDim.x * (blockDim.x >> 5) * 2;  // blocks at one pair per warp
+  if (total <= one) rs_solve<1>(P, s_end, total, sweeps, bar);
+  else if (total <= 2 * one) rs_solve<2>(P, s_end, total, sweeps, bar);
+  else if (total <= 4 * one) rs_solve<4>(P, s_end, total, sweeps, bar);
+  else rs_solve<8>(P, s_end, total, sweeps, bar);
 }
 
 // The sweeps of one level transposed (k_adj_jacobi for each, last to first).
@@ -363,8 +378,8 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 1)
       if (k >= pairs) break;
       const uint4 r = rest.at(k);
       Halo hv;
-      rs_load(src, q[k], r, h, hv);
-      rs_fix<true>(q[k], r, hv);
+      rs_load(src, q[k], r, hv);
+      rs_fix<true>(q[k], r, h, hv);
       float2 s[2];
       rs_sums(q[k], hv, h, s);
       div6_pairs(s);
@@ -446,10 +461,7 @@ bool launch_resident_solve(const SolveBatch &P, int sweeps, int sms, cudaStream_
   for (int m = 0; m < P.n; m++)
     if (P.lev[m] >= 0) blocks += P.d[m].g.budget[P.lev[m]];
   if (sweeps <= 0 || blocks > resident_blocks(sms, 8)) return false;
-  if (blocks <= resident_blocks(sms, 1)) return resident_launch<1>(k_resident_solve<1>, blocks, sms, st, P, sweeps);
-  if (blocks <= resident_blocks(sms, 2)) return resident_launch<2>(k_resident_solve<2>, blocks, sms, st, P, sweeps);
-  if (blocks <= resident_blocks(sms, 4)) return resident_launch<4>(k_resident_solve<4>, blocks, sms, st, P, sweeps);
-  return resident_launch<8>(k_resident_solve<8>, blocks, sms, st, P, sweeps);
+  return resident_launch<8>(k_resident_solve, blocks, sms, st, P, sweeps);
 }
 bool launch_resident_adjoint(const Dev &D, int level, int sweeps, float *lp0, float *lp1, float *ld, int sms,
                              cudaStream_t st) {
