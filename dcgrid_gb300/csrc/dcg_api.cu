@@ -323,7 +323,14 @@ int dcg_get_field(dcg_sim *s, int32_t field, float *dst, int32_t where) {
   const size_t cells = field_cells(s), n = cells * sizeof(float);
   int rc;
   const float *src = static_cast<const float *>(r.p);
-  if (r.mode) {  // 16-bit storage: widen into an FP32 staging buffer
+  if (r.mode) {  // 16-bit storage: widen into the buffer when it is this GPU's own memory, else into an FP32 staging buffer
+    cudaPointerAttributes at{};
+    if (where == DCG_DEVICE && cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+        at.device == s->device) {
+      launch_h16_to_f32(static_cast<const uint16_t *>(r.p), dst, (long long)cells, r.mode, s->stream);
+      if ((rc = s->check_launch("get_field"))) return rc;
+      return s->sync("get_field");
+    }
     if (!s->conv_tmp && (rc = s->alloc(&s->conv_tmp, cells))) return rc;
     launch_h16_to_f32(static_cast<const uint16_t *>(r.p), s->conv_tmp, (long long)cells, r.mode, s->stream);
     src = s->conv_tmp;

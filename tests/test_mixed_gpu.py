@@ -72,3 +72,29 @@ def test_bf16_error_is_reported():
     err = rel_errors(capi.PRECISION_MIXED, 30)
     print("bf16 relative L2 error vs FP64 oracle after 30 steps:", {k: f"{v:.2e}" for k, v in err.items()})
     assert err["density"] < 2e-2  # bf16 storage: a few 1e-3; reported, not within the 1e-3 bar
+
+
+@pytest.mark.parametrize("precision", [capi.PRECISION_MIXED, capi.PRECISION_MIXED_FP16])
+def test_fields_into_device_buffers(precision):
+    """A CUDA buffer, aligned or not, receives what the host copy does, bit for
+    bit: subnormals, infinities and NaN of the 16-bit format included."""
+    import torch
+    from dcgrid_gb300 import Simulation
+    p = scenarios.plume(32, 32, 40, None, 2, 2)
+    p.precision = precision
+    s = Simulation(p)
+    n = s.num_cells
+    bits = np.resize(np.arange(65536, dtype=np.uint16), n)
+    values = bits.view(np.float16).astype(np.float32) if precision == capi.PRECISION_MIXED_FP16 \
+        else (bits.astype(np.uint32) << 16).view(np.float32)
+    s.set_field("density", values)
+    host = s.get_field("density")
+    assert np.array_equal(host[~np.isnan(values)], values[~np.isnan(values)])
+    for offset in (0, 1, 4):
+        whole = torch.full((n + 8,), 7.0, dtype=torch.float32, device="cuda")
+        part = whole[offset:offset + n]
+        torch.cuda.synchronize()
+        s.get_field("density", out=part)
+        got = whole.cpu().numpy()
+        assert np.array_equal(got[offset:offset + n].view(np.uint32), host.view(np.uint32))
+        assert (got[:offset] == 7).all() and (got[offset + n:] == 7).all()
