@@ -110,33 +110,25 @@ struct dcg_batch {
   }
 
   // ------------------------------------------------------------ stage launches
-  // the members a stage launch covers: all, or the listed ones
-  std::vector<int> all_members() const {
-    std::vector<int> v(n());
-    for (int i = 0; i < n(); i++) v[i] = i;
-    return v;
-  }
-  void cells(int stage) { cells(stage, all_members(), stream); }
-  void cells(int stage, const std::vector<int> &mem, cudaStream_t st) {
-    for (size_t g = 0; g < mem.size(); g += BMAX) {
+  void cells(int stage) {
+    for (int g = 0; g < n(); g += BMAX) {
       CellBatch P{};
-      P.n = (int)std::min<size_t>(BMAX, mem.size() - g);
-      for (int i = 0; i < P.n; i++) P.d[i] = m[mem[g + i]]->D;
-      launch_cells_batch(stage, P, stage == 5 ? 1 : tune.tile[stage], st, tune.persistent != 0);
+      P.n = std::min(BMAX, n() - g);
+      for (int i = 0; i < P.n; i++) P.d[i] = m[g + i]->D;
+      launch_cells_batch(stage, P, stage == 5 ? 1 : tune.tile[stage], stream, tune.persistent != 0);
     }
   }
   // field: 0 velocity, 1 scalars, 2 divergence, 3 velocity and scalars
-  void restrict_fields(int field) { restrict_fields(field, all_members(), stream); }
-  void restrict_fields(int field, const std::vector<int> &mem, cudaStream_t st) {
+  void restrict_fields(int field) {
     int maxl = 0;
-    for (int i : mem) maxl = std::max(maxl, m[i]->D.g.levels);
+    for (int i = 0; i < n(); i++) maxl = std::max(maxl, m[i]->D.g.levels);
     for (int level = 0; level < maxl - 1; level++)
-      for (size_t g = 0; g < mem.size(); g += BMAX) {
+      for (int g = 0; g < n(); g += BMAX) {
         RestrictBatch P{};
-        P.n = (int)std::min<size_t>(BMAX, mem.size() - g);
+        P.n = std::min(BMAX, n() - g);
         P.level = level;
         for (int i = 0; i < P.n; i++) {
-          const dcg_sim *s = m[mem[g + i]];
+          const dcg_sim *s = m[g + i];
           P.d[i] = s->D;
           FieldList &fl = P.fl[i];
           if (field == 0 || field == 3) {
@@ -156,7 +148,7 @@ struct dcg_batch {
             fl.f[0] = s->D.div;
           }
         }
-        launch_restrict_batch(P, st);
+        launch_restrict_batch(P, stream);
       }
   }
   // FP64 defect correction after the cascade (dcg_sim::defect_correct for
@@ -652,7 +644,12 @@ int dcg_batch_create(int32_t n, const dcg_params *params, dcg_batch **out) {
     b->S2.push_back(S2);
   }
   b->cl_size = cluster_solve_size();
-  for (int k = 0; k < 4; k++) b->tune.tile[k] = 4;
+  // until a schedule is set or tuned: the staged cell stages, which fuse the
+  // pressure application into the scalar advection (8 members of up to 160^3,
+  // us per step and read-outs: 944 with four blocks per CTA, 815 staged; 18 of
+  // up to 64^3 872 both)
+  for (int k = 0; k < 4; k++) b->tune.tile[k] = 1;
+  b->tune.persistent = 1;
   b->tune.solve_cache = 4;
   b->tune.solve_ctas_per_sm = 0;
   b->tune.solve_barrier = 1;
