@@ -87,6 +87,7 @@ struct SolveBatch {
   unsigned long long arena[BMAX];  // first cell of member s in the arenas
   int lev[BMAX];
   long long cl_max[BMAX];
+  long long res_max;  // the resident solve has taken the launch if no more blocks than this remain
   Dev d[BMAX];
 };
 // Cluster solve (k_cascade.cu): member s's levels hi[s] down to lo[s], one
@@ -122,8 +123,11 @@ bool solve_variant_valid(int cache);
 void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cache, cudaStream_t st);
 
 // k_resident.cu: the same solve, and a level's sweeps transposed, with the
-// cells in registers; false: too many blocks (or a form that they do not take)
-bool launch_resident_solve(const SolveBatch &P, int sweeps, int sms, cudaStream_t st);
+// cells in registers; false: too many blocks (or a form that they do not take).
+// Where the budgets are too large and the blocks allocated may not be, the
+// resident solve is launched, the device decides, P.res_max tells the general
+// solve, and the answer is false too.
+bool launch_resident_solve(SolveBatch &P, int sweeps, int sms, cudaStream_t st);
 bool launch_resident_adjoint(const Dev &D, int level, int sweeps, float *lp0, float *lp1, float *ld, int sms,
                              cudaStream_t st);
 

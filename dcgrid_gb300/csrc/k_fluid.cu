@@ -930,7 +930,8 @@ __global__ void __launch_bounds__(256, NB ? MB : DCG_SOLVE_MINB)
   }
   __syncthreads();
   const long long total = s_end[P.n - 1];
-  if (total == 0) return;  // the cluster solve took every level: the same in every CTA
+  // the cluster solve took every level, or the resident solve the rest: the same in every CTA
+  if (total == 0 || (total >> 6) <= P.res_max) return;
   const unsigned nctas = gridDim.x;
   const long long stride = (long long)nctas * 256;
   const long long first = (long long)blockIdx.x * 256 + t;

@@ -309,9 +309,10 @@ __global__ void __launch_bounds__(RS_WARPS * 32, 1) k_resident_solve(const __gri
   }
   __syncthreads();
   const long long total = s_end[P.n - 1];
-  if (total == 0) return;  // the cluster solve took every level: the same in every CTA
-  GridBarrier bar(P.bar, P.err, gridDim.x);
   const long long one = (long long)gridDim.x * (blockDim.x >> 5) * 2;  // blocks at one pair per warp
+  // the cluster solve took every level, or the general solve will: the same in every CTA
+  if (total == 0 || total > 8 * one) return;
+  GridBarrier bar(P.bar, P.err, gridDim.x);
   if (total <= one) rs_solve<1>(P, s_end, total, sweeps, bar);
   else if (total <= 2 * one) rs_solve<2>(P, s_end, total, sweeps, bar);
   else if (total <= 4 * one) rs_solve<4>(P, s_end, total, sweeps, bar);
@@ -456,12 +457,20 @@ static bool resident_launch(Kernel kernel, long long blocks, int sms, cudaStream
 // blocks that CTAs with k pairs per warp hold
 static long long resident_blocks(int sms, int k) { return (long long)sms * RS_WARPS * k * 2; }
 
-bool launch_resident_solve(const SolveBatch &P, int sweeps, int sms, cudaStream_t st) {
-  long long blocks = 0;
-  for (int m = 0; m < P.n; m++)
-    if (P.lev[m] >= 0) blocks += P.d[m].g.budget[P.lev[m]];
-  if (sweeps <= 0 || blocks > resident_blocks(sms, 8)) return false;
-  return resident_launch<8>(k_resident_solve, blocks, sms, st, P, sweeps);
+bool launch_resident_solve(SolveBatch &P, int sweeps, int sms, cudaStream_t st) {
+  long long blocks = 0, always = 0;  // budgets, and those of levels allocated in full
+  for (int m = 0; m < P.n; m++) {
+    const Geom &g = P.d[m].g;
+    if (P.lev[m] < 0) continue;
+    blocks += g.budget[P.lev[m]];
+    if (g.budget[P.lev[m]] == g.full[P.lev[m]]) always += g.budget[P.lev[m]];
+  }
+  const long long most = resident_blocks(sms, 8);
+  P.res_max = 0;
+  if (sweeps <= 0 || always > most) return false;
+  const bool done = resident_launch<8>(k_resident_solve, blocks, sms, st, P, sweeps);
+  if (done && blocks > most) P.res_max = most;
+  return done && blocks <= most;
 }
 bool launch_resident_adjoint(const Dev &D, int level, int sweeps, float *lp0, float *lp1, float *ld, int sms,
                              cudaStream_t st) {

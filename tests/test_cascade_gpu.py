@@ -217,3 +217,23 @@ def test_transposed_projection_matches_fp64(g, blocks, iters, compat):
     for d in range(3):
         a, b = got[d * nc:(d + 1) * nc], want[d * nc:(d + 1) * nc]
         assert np.linalg.norm(a - b) <= 1e-4 * np.linalg.norm(b)
+
+
+# a budget beyond what the chip holds: the blocks allocated, known on the device
+# only, send the level to the resident solve (few of them) or to the general one
+@pytest.mark.parametrize("many", [False, True])
+def test_budget_beyond_the_resident_solve_bitexact(many):
+    p = scenarios.plume(160, 160, 128, 20 * 20 * 16 + 46601, 2, 4)
+    if not many:  # refined around the source only
+        p.refine_criterion = capi.REFINE_FIELDS
+        p.refine_threshold, p.vort_threshold, p.grad_threshold = 1.0, 0.5, 0.05
+        p.src_radius = 60.0
+    g, o = pair(p, 0.5 if many else 0.0)
+    assert 38912 < g.info.budget[0] < g.info.full_blocks[0]
+    for s in (g, o):
+        s.step(3)
+        s.project_local()
+    g.sync()
+    load = g.get_topology()["load"][0]
+    assert load > 38912 if many else 1024 < load <= 38912
+    same(g, o)
