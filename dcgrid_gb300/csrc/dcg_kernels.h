@@ -176,10 +176,11 @@ void launch_dense_solve(const Dev *d, const int *lev, int n, int prolong, int sw
 
 // Host schedule of a cascade over any number of simulations: every level of
 // every member, coarse to fine, each by the solver that suits it. The levels
-// whose budget a cluster holds go to the cluster solve, runs of them in one
-// launch; larger levels that are allocated in full, in raster order, to the
-// dense solve; a larger sparse level goes to the cluster solve too while its
-// allocated blocks fit (known on the device only), else to `general`, which is
+// whose budget suits a cluster go to the cluster solve, runs of them in one
+// launch; levels that are allocated in full, in raster order, to the dense
+// solve where together they have kDenseBlocks; a larger sparse level goes to
+// the cluster solve too while its allocated blocks fit (known on the device
+// only), else to `general` (the resident solve or the staged one), which is
 // launched behind it and leaves what the cluster solve took.
 struct Cascade {
   int csize = 0;  // cluster size of the device (0: no cluster solve)

@@ -898,6 +898,7 @@ __device__ __forceinline__ void solve_pipelined(const SolveBatch &P, const long 
 
 // One round of the batched cascade: level P.lev[m] of every member m that has
 // one and whose level the cluster solve leaves (more than P.cl_max[m] blocks),
+// unless the resident solve takes them (P.res_max blocks or fewer):
 // optional prolongation from the member's parent level, then `sweeps` Jacobi
 // sweeps over the concatenated cells of all members, separated by grid
 // barriers. Member m's cells of the level

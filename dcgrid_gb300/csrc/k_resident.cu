@@ -12,9 +12,9 @@
 // blocks on the shuffles and the halo's sectors. Copying blocks and halos to
 // shared tiles in every sweep (k_level_solve_batch, which larger levels need)
 // took 3.1 us per sweep of 4096 blocks, 3.9 of 8192 and 7.7 of 32768; here they
-// take 2.0, 2.4 and 5.7. A cluster (k_cascade.cu) takes 1.4 for 1024 blocks and
-// 2.05 for 2048, here 1.8 and 1.9 and a launch: the line between them stays at
-// what a cluster holds.
+// take 2.0, 2.4 and 5.8. A cluster (k_cascade.cu) takes 1.4 for 1024 blocks and
+// 2.05 for 2048, here 1.8 and 1.9 and a launch: the line lies where a cluster
+// has one group of blocks per warp, 1024.
 #include "dcg_dev.cuh"
 #include "dcg_kernels.h"
 
@@ -435,11 +435,15 @@ template <int K, class Kernel, class... Args>
 static bool resident_launch(Kernel kernel, long long blocks, int sms, cudaStream_t st, const Args &...args) {
   const size_t smem = Rests<K>::kBytes;
   int occ = 0;
+  // a device that refuses the launch has the other solvers: no error is left behind
+  auto ok = [](cudaError_t e) {
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
+  };
   if (smem > 48 * 1024 &&
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      !ok(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)))
     return false;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, RS_WARPS * 32, smem) != cudaSuccess || occ < 1)
-    return false;
+  if (!ok(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, RS_WARPS * 32, smem)) || occ < 1) return false;
   // as many warps as hold the blocks in one pair each, up to the CTA's limit
   const long long pairs = (blocks + 1) / 2, warps = (pairs + sms - 1) / sms;
   cudaLaunchConfig_t cfg = {};
@@ -452,7 +456,7 @@ static bool resident_launch(Kernel kernel, long long blocks, int sms, cudaStream
   attr.val.cooperative = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...) == cudaSuccess;
+  return ok(cudaLaunchKernelEx(&cfg, kernel, args...));
 }
 // blocks that CTAs with k pairs per warp hold
 static long long resident_blocks(int sms, int k) { return (long long)sms * RS_WARPS * k * 2; }
