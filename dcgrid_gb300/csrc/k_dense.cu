@@ -384,12 +384,12 @@ static void dn_plan(DensePass &P, int T, int sms) {
   }
 }
 
-template <int T, bool UNI, bool EDGE> static cudaError_t dn_launch(const DensePass &P, cudaStream_t st) {
-  static const cudaError_t ok =
-      cudaFuncSetAttribute(k_dense_pass<T, UNI, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dn_smem<T>());
-  if (ok != cudaSuccess) return ok;
-  k_dense_pass<T, UNI, EDGE><<<(unsigned)P.end[P.n - 1], dn_threads<T>(), dn_smem<T>(), st>>>(P);
-  return cudaSuccess;
+// The opt-in to this much shared memory belongs to the current device, so every
+// launch asks for it; a refusal is left to the caller's launch check.
+template <int T, bool UNI, bool EDGE> static void dn_launch(const DensePass &P, cudaStream_t st) {
+  if (cudaFuncSetAttribute(k_dense_pass<T, UNI, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dn_smem<T>()) ==
+      cudaSuccess)
+    k_dense_pass<T, UNI, EDGE><<<(unsigned)P.end[P.n - 1], dn_threads<T>(), dn_smem<T>(), st>>>(P);
 }
 
 // sweeps (even, > 0) of the levels: src -> dst with dst2 = the iterate before

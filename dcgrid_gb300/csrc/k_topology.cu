@@ -1020,11 +1020,12 @@ template <int PHASE> __global__ void __launch_bounds__(DC_THREADS, 1) k_decide(c
     if (threadIdx.x == 0) finish_refines_body(D, 0, 1);
   }
 }
+// the shared-memory opt-in belongs to the current device, so every launch asks
+// for it; a refusal is left to the caller's launch check
 static void launch_decide(int phase, const DecideP &P, cudaStream_t st) {
   if (phase == 0) {
-    static const cudaError_t ok = cudaFuncSetAttribute(k_decide<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SMEM);
-    (void)ok;
-    k_decide<0><<<P.n, DC_THREADS, DC_SMEM, st>>>(P);
+    if (cudaFuncSetAttribute(k_decide<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, DC_SMEM) == cudaSuccess)
+      k_decide<0><<<P.n, DC_THREADS, DC_SMEM, st>>>(P);
   } else {
     k_decide<1><<<P.n, DC_THREADS, 0, st>>>(P);
   }

@@ -438,10 +438,13 @@ void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, bool 
     const int top = U.levels - 1;
     int l = top;
     while (l >= 0 && ucells(U, l) <= SB_CELLS) l--;
-    if (l < top) {  // the levels that one CTA holds
-      static const cudaError_t ok = cudaFuncSetAttribute(k_u_small, cudaFuncAttributeMaxDynamicSharedMemorySize, SB_SMEM);
-      if (ok == cudaSuccess) k_u_small<<<1, SB_THREADS, SB_SMEM, st>>>(U, top, l + 1, 2 * top_pairs, 2 * pairs);
-      else l = top;
+    if (l < top) {  // the levels that one CTA holds; the shared-memory opt-in is the current device's
+      if (cudaFuncSetAttribute(k_u_small, cudaFuncAttributeMaxDynamicSharedMemorySize, SB_SMEM) == cudaSuccess) {
+        k_u_small<<<1, SB_THREADS, SB_SMEM, st>>>(U, top, l + 1, 2 * top_pairs, 2 * pairs);
+      } else {
+        cudaGetLastError();  // a launch per sweep takes its place
+        l = top;
+      }
     }
     for (; l >= 0; l--) u_sweeps(U, l, 2 * (l == top ? top_pairs : pairs), l == top, sms, st);
   }
