@@ -330,25 +330,14 @@ struct dcg_batch {
       auto it = graphs.find(key);
       int rc;
       if (it == graphs.end()) {
-        cudaGraph_t g = nullptr;
-        if ((rc = cuda(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "capture"))) return rc;
-        step_once();
-        if ((rc = cuda(cudaStreamEndCapture(stream, &g), "end capture"))) return rc;
-        size_t nn = 0;
-        if (cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {
-          std::vector<cudaGraphNode_t> nodes(nn);
-          cudaGraphGetNodes(g, nodes.data(), &nn);
-          long long nk = 0;
-          for (auto nd : nodes) {
-            cudaGraphNodeType t;
-            if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) nk++;
-          }
-          kernels_per_step = nk;
-        }
         cudaGraphExec_t ge = nullptr;
-        rc = cuda(cudaGraphInstantiate(&ge, g, 0), "instantiate");
-        cudaGraphDestroy(g);
-        if (rc) return rc;
+        if ((rc = cuda(capture_graph(stream, [&] { step_once(); }, &ge, &kernels_per_step), "step graph"))) {
+          if (m[0]->vpar * 2 + m[0]->qpar != key) {  // nothing has run
+            flip_v();
+            flip_q();
+          }
+          return rc;
+        }
         graphs[key] = ge;
         // step_once() advanced the members' parities while capturing
         if ((rc = cuda(cudaGraphLaunch(ge, stream), "graph launch"))) return rc;

@@ -23,6 +23,34 @@ namespace {
 
 int idiv_up(int a, int b) { return (a % b != 0) ? (a / b + 1) : (a / b); }
 
+// Captures the launches of fn() on the stream as a graph, its kernels counted.
+// A launch that the device refuses has no node in the graph, so its error is
+// looked for before the graph is kept: none is made then.
+template <class F> cudaError_t capture_graph(cudaStream_t stream, F fn, cudaGraphExec_t *out, long long *kernels) {
+  cudaGraph_t g = nullptr;
+  cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) {
+    fn();
+    const cudaError_t refused = cudaGetLastError();
+    e = cudaStreamEndCapture(stream, &g);
+    if (refused != cudaSuccess) e = refused;
+  }
+  size_t nn = 0;
+  if (e == cudaSuccess && cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {
+    std::vector<cudaGraphNode_t> nodes(nn);
+    cudaGraphGetNodes(g, nodes.data(), &nn);
+    *kernels = 0;
+    for (auto nd : nodes) {
+      cudaGraphNodeType t;
+      if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) ++*kernels;
+    }
+  }
+  if (e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (e != cudaSuccess) cudaGetLastError();  // returned here, not by a later check
+  return e;
+}
+
 }  // namespace
 
 namespace dcg {
@@ -104,7 +132,6 @@ struct dcg_sim {
   int device = 0, sms = 148;
   std::vector<void *> allocs;
   size_t bytes = 0;
-  bool failed = false;
   long long steps = 0;
 
   // adaptive
@@ -172,7 +199,6 @@ struct dcg_sim {
   int cuda(cudaError_t e, const char *what) {
     if (e == cudaSuccess) return DCG_OK;
     err = std::string(what) + ": " + cudaGetErrorString(e);
-    failed = true;
     return DCG_E_CUDA;
   }
   // plan_only: creation only adds up the device bytes it would allocate
@@ -791,43 +817,30 @@ struct dcg_sim {
     }
   }
 
+  void flip() {
+    vpar ^= 1;
+    qpar ^= 1;
+    bind_parity();
+  }
   int step(int n) {
     for (int i = 0; i < n; i++) {
       if (use_graphs) {
         const int key = vpar * 2 + qpar;
         auto it = graphs.find(key);
         if (it == graphs.end()) {
-          cudaGraph_t g = nullptr;
-          int rc;
-          if ((rc = cuda(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "capture"))) return rc;
-          step_once();
-          if ((rc = cuda(cudaStreamEndCapture(stream, &g), "end capture"))) return rc;
-          size_t nn = 0;
-          if (cudaGraphGetNodes(g, nullptr, &nn) == cudaSuccess && nn > 0) {
-            std::vector<cudaGraphNode_t> nodes(nn);
-            cudaGraphGetNodes(g, nodes.data(), &nn);
-            long long nk = 0;
-            for (auto nd : nodes) {
-              cudaGraphNodeType t;
-              if (cudaGraphNodeGetType(nd, &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) nk++;
-            }
-            kernels_per_step = nk;
-          }
           cudaGraphExec_t ge = nullptr;
-          if ((rc = cuda(cudaGraphInstantiate(&ge, g, 0), "instantiate"))) {
-            cudaGraphDestroy(g);
+          int rc;
+          if ((rc = cuda(capture_graph(stream, [&] { step_once(); }, &ge, &kernels_per_step), "step graph"))) {
+            if (vpar * 2 + qpar != key) flip();  // nothing has run
             return rc;
           }
-          cudaGraphDestroy(g);
           graphs[key] = ge;
           // step_once() advanced the buffer parities while capturing
           if ((rc = cuda(cudaGraphLaunch(ge, stream), "graph launch"))) return rc;
         } else {
           int rc;
           if ((rc = cuda(cudaGraphLaunch(it->second, stream), "graph launch"))) return rc;
-          vpar ^= 1;
-          qpar ^= 1;
-          bind_parity();
+          flip();
         }
       } else {
         step_once();

@@ -178,7 +178,8 @@ cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t a, cudaEvent_t b) {
   *ms = (float)(*reinterpret_cast<double *>(b) - *reinterpret_cast<double *>(a));
   return cudaSuccess;
 }
-cudaError_t cudaStreamBeginCapture(cudaStream_t, enum cudaStreamCaptureMode) {
+cudaError_t cudaStreamBeginCapture(cudaStream_t s, enum cudaStreamCaptureMode) {
+  if (!s) return fail(cudaErrorStreamCaptureUnsupported);  // the legacy stream
   g_capture = new std::vector<std::string>;
   return cudaSuccess;
 }

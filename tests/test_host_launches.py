@@ -1,5 +1,6 @@
 """The library's host code (launch attributes, routes, step graphs) on the CPU,
 with a runtime that records the launches (tests/fake_gpu.py)."""
+import numpy as np
 import pytest
 
 from dcgrid_gb300 import capi
@@ -27,3 +28,43 @@ def test_large_shared_memory_on_every_device(fake, scene, mode, kernel):  # noqa
         s.step(1)
         s.project()
         assert any(kernel in n for n in fake.launches()), device
+
+
+def small_scene():
+    return scenarios.plume(32, 32, 32, None, 2, 4)
+
+
+@pytest.mark.parametrize("batch", [False, True])
+def test_refused_launch_leaves_no_step_graph(fake, batch):  # noqa: F811
+    """A launch that the device refuses has no node in the graph under capture:
+    every step reports it, none is replayed without it, and the state is the one
+    before the step."""
+    from dcgrid_gb300 import Batch, DcgError, Simulation
+
+    def handle():
+        h = Batch([small_scene(), small_scene()]) if batch else Simulation(small_scene())
+        return h, (h[0] if batch else h)
+    h, sim = handle()
+    velocity = np.arange(sim.num_cells, dtype=np.float32)
+    sim.set_field("vel_x", velocity)
+    fake.refuse("k_cluster_solve")
+    fake.launches()
+    for capture in (True, True, True, False):
+        if not capture:  # the legacy stream cannot be captured
+            fake.refuse("")
+            h.set_stream(0)
+        with pytest.raises(DcgError) as e:
+            h.step(1)
+        assert e.value.code == capi.DCG_E_CUDA
+        assert fake.launches() == []
+        assert np.array_equal(sim.get_field("vel_x"), velocity)
+    assert sim.stats().steps == 0
+    h.set_stream(1)
+    fake.launches()
+    h.step(2)
+    got = fake.launches()
+    assert any("k_cluster_solve" in n for n in got)
+    fresh = handle()[0]
+    fake.launches()
+    fresh.step(2)
+    assert got == fake.launches()
