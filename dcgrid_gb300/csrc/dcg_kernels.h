@@ -194,7 +194,7 @@ struct Cascade {
   long long limit() const { return csize > 0 ? cluster_solve_blocks(csize) : 0; }
   // general(members, levels, limit, round): solve levels[i] of members[i]
   // unless at most `limit` of its blocks are allocated
-  // raster[i]: member i's full levels lie in raster order; only >= 0: that level alone
+  // raster[i]: member i's full levels are allocated, in raster order; only >= 0: that level alone
   template <class General> void run(const Dev *d, const char *raster, int n, General general, int only = -1) const;
 };
 

@@ -96,8 +96,10 @@ void Cascade::run(const Dev *d, const char *raster, int n, General general, int 
         gm.push_back(i);
         gl.push_back(l);
         cur[i] = l - 1;
-        if (lim > 0 && g.budget[l] < g.full[l]) blocks = lim;
-        else l++;  // allocated in full: never fits a cluster
+        // in full (a budget that covers the grid is not enough: a topology from
+        // outside may hold fewer blocks): never fits a cluster
+        if (lim == 0 || (g.budget[l] == g.full[l] && raster[i])) l++;
+        else blocks = lim;
       }
       if (l <= top) {
         mem.push_back(i);
@@ -171,8 +173,8 @@ struct dcg_sim {
   // cannot be formed on the device, and the per-level kernel takes its place)
   int ls_grid_staged = 0;
   int cl_size = 0;         // cluster size of the small levels' solve (0: none)
-  // the full levels lie in raster order, as created (a caller's topology or
-  // state may say otherwise: check_raster)
+  // the full levels are allocated in full and lie in raster order, as created (a
+  // caller's topology or state may say otherwise: check_raster)
   char raster = 1;
   // level solve of single simulations: pipelined staged sweeps, two tile buffers,
   // block descriptions cached in 3 x 8 KB of shared memory when they fit.

@@ -58,8 +58,36 @@ void run(const std::string &name) {
     if (name.find(c.first) != std::string::npos) ms = c.second;
   g_clock += ms;
 }
+// the heads of two kernels' parameters: dcg::ClusterSolve and dcg::SolveBatch
+struct ClusterArgs {
+  int n, csize, sweeps, prolong;
+  long long limit;
+  int hi[16], lo[16];
+};
+struct SolveArgs {
+  int n, prolong;
+  void *planes[6];
+  unsigned long long arena[16];
+  int lev[16];
+  long long cl_max[16], res_max;
+};
+// which levels a solver takes, behind its name: ":highest-lowest" of every
+// member, or ":level>blocks that it leaves", and the launch's "<blocks that it leaves"
+std::string levels_of(const std::string &name, void **args) {
+  std::string t;
+  if (name.find("k_cluster_solve") != std::string::npos) {
+    const ClusterArgs &a = *static_cast<const ClusterArgs *>(args[0]);
+    for (int i = 0; i < a.n; i++) t += ":" + std::to_string(a.hi[i]) + "-" + std::to_string(a.lo[i]);
+  }
+  if (name.find("k_resident_solve") != std::string::npos || name.find("k_level_solve_batch") != std::string::npos) {
+    const SolveArgs &a = *static_cast<const SolveArgs *>(args[0]);
+    for (int i = 0; i < a.n; i++) t += ":" + std::to_string(a.lev[i]) + ">" + std::to_string(a.cl_max[i]);
+    t += "<" + std::to_string(a.res_max);
+  }
+  return t;
+}
 cudaError_t launch(const void *f, size_t smem, void **args) {
-  const std::string &name = name_of(f);
+  const std::string name = name_of(f) + levels_of(name_of(f), args);
   for (auto &r : g_refused)
     if (name.find(r) != std::string::npos) return fail(cudaErrorLaunchOutOfResources);
   if (smem > 48 * 1024) {

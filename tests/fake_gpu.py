@@ -41,7 +41,8 @@ class Fake:
         return p.value
 
     def launches(self):
-        """mangled names of the kernels launched since the last call"""
+        """the kernels launched since the last call: mangled names, the solvers
+        with their levels (levels_of in fake_cudart.cpp)"""
         names = self.lib.fake_log().decode().split()
         self.lib.fake_clear()
         return names

@@ -68,3 +68,20 @@ def test_refused_launch_leaves_no_step_graph(fake, batch):  # noqa: F811
     fake.launches()
     fresh.step(2)
     assert got == fake.launches()
+
+
+def test_partly_allocated_full_level_is_solved(fake):  # noqa: F811
+    """A topology from outside may hold fewer blocks of a level than its budget,
+    which covers the block grid: the device counts them, so the cluster solve has
+    to be launched over that level as over a sparse one."""
+    from dcgrid_gb300 import Simulation
+    s = Simulation(scenarios.plume(64, 64, 64, 512 + 4096, 2, 4))
+    assert s.info.budget[0] == s.info.full_blocks[0] == 4096  # more than a cluster holds
+    fake.launches()
+    s.project()
+    assert [n.split(":")[1] for n in fake.launches() if "k_cluster_solve" in n] == ["1-1"]
+    fake.raster_bad(True)
+    s.set_topology(s.get_topology())
+    fake.launches()
+    s.project()
+    assert [n.split(":")[1] for n in fake.launches() if "k_cluster_solve" in n] == ["1-0"]
