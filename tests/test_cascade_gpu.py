@@ -237,3 +237,21 @@ def test_budget_beyond_the_resident_solve_bitexact(many):
     load = g.get_topology()["load"][0]
     assert load > 38912 if many else 1024 < load <= 38912
     same(g, o)
+
+
+def test_tiles_beyond_the_box_cost_no_division_tests():
+    """Full levels whose tiles overhang the box (39936 blocks) and whose tiles
+    cover it exactly (45056): the dense passes' time per sweep follows the tiles.
+    The overhang's own work is an eighth here; a warp that takes the division's
+    component-wise test in every sweep made it 1.42 times the larger level's."""
+    from dcgrid_gb300 import Simulation
+    best = []
+    for z in (39, 44):
+        s = Simulation(scenarios.plume(128, 128, 4 * z, 32 * 32 * z, 1, 100))
+        s.add_velocity_noise(1, 0.5)
+        s.step(2)
+        s.sync()
+        best.append(min(s.time_kernel(4, 0, 5)[0] for _ in range(7)))
+        s.close()
+    print("us per sweep:", [round(10 * t, 2) for t in best])
+    assert best[0] < 1.25 * best[1]
