@@ -128,6 +128,7 @@ void launch_level_solve_batch(const SolveBatch &P, int sweeps, int grid, int cac
 // resident solve is launched, the device decides, P.res_max tells the general
 // solve, and the answer is false too.
 bool launch_resident_solve(SolveBatch &P, int sweeps, int sms, cudaStream_t st);
+long long resident_solve_blocks(int sms);  // the most blocks that it holds
 bool launch_resident_adjoint(const Dev &D, int level, int sweeps, float *lp0, float *lp1, float *ld, int sms,
                              cudaStream_t st);
 
@@ -178,19 +179,21 @@ void launch_dense_solve(const Dev *d, const int *lev, int n, int prolong, int sw
 // every member, coarse to fine, each by the solver that suits it. The levels
 // whose budget suits a cluster go to the cluster solve, runs of them in one
 // launch; levels that are allocated in full, in raster order, to the dense
-// solve where together they have kDenseBlocks; a larger sparse level goes to
-// the cluster solve too while its allocated blocks fit (known on the device
-// only), else to `general` (the resident solve or the staged one), which is
-// launched behind it and leaves what the cluster solve took.
+// solve where together they have more blocks than the resident solve holds; a
+// larger sparse level goes to the cluster solve too while its allocated blocks
+// fit (known on the device only), else to `general` (the resident solve or the
+// staged one), which is launched behind it and leaves what the cluster solve
+// took.
 struct Cascade {
   int csize = 0;  // cluster size of the device (0: no cluster solve)
   int sms = 148;
   int sweeps = 0, prolong = 1;
   cudaStream_t st = nullptr;
-  // blocks that make the dense solve the faster one: more than the resident
-  // solve holds on 152 SMs (us per sweep of 36864 blocks: dense 11.4, resident
-  // 6.2; of 65536: dense 8.5, k_level_solve_batch 13.0)
-  static constexpr long long kDenseBlocks = 38913;
+  // from this many blocks on the dense solve takes full levels: one more than
+  // the resident solve holds, 38913 on 152 SMs (us per sweep, dense, resident,
+  // k_level_solve_batch: 32768 blocks 8.1, 5.8, 7.7; 38912 8.4, 6.5, 9.1; 39936
+  // 9.4, -, 8.9; 40960 8.4 to 8.6, -, 9.3; 45056 8.4, -, 10.0; 65536 8.0, -, 13.0)
+  long long dense_blocks() const { return resident_solve_blocks(sms) + 1; }
   long long limit() const { return csize > 0 ? cluster_solve_blocks(csize) : 0; }
   // general(members, levels, limit, round): solve levels[i] of members[i]
   // unless at most `limit` of its blocks are allocated

@@ -73,7 +73,7 @@ void Cascade::run(const Dev *d, const char *raster, int n, General general, int 
         dm.push_back(i);
         blocks += d[i].g.budget[cur[i]];
       }
-    if (blocks >= kDenseBlocks) {
+    if (blocks >= dense_blocks()) {
       launch_dense_solve(dd.data(), dl.data(), (int)dd.size(), prolong, sweeps, sms, st);
       for (int i : dm) cur[i]--;
       continue;
@@ -90,7 +90,7 @@ void Cascade::run(const Dev *d, const char *raster, int n, General general, int 
       cur[i] = l;
       if (l < last) {
         l = last;
-      } else if (full(i) && raster[i] && g.budget[l] >= kDenseBlocks && sweeps > 0) {
+      } else if (full(i) && raster[i] && g.budget[l] >= dense_blocks() && sweeps > 0) {
         l++;  // the dense solve's, next
       } else {
         gm.push_back(i);

@@ -460,6 +460,7 @@ static bool resident_launch(Kernel kernel, long long blocks, int sms, cudaStream
 }
 // blocks that CTAs with k pairs per warp hold
 static long long resident_blocks(int sms, int k) { return (long long)sms * RS_WARPS * k * 2; }
+long long resident_solve_blocks(int sms) { return resident_blocks(sms, 8); }
 
 bool launch_resident_solve(SolveBatch &P, int sweeps, int sms, cudaStream_t st) {
   long long blocks = 0, always = 0;  // budgets, and those of levels allocated in full
@@ -469,7 +470,7 @@ bool launch_resident_solve(SolveBatch &P, int sweeps, int sms, cudaStream_t st) 
     blocks += g.budget[P.lev[m]];
     if (g.budget[P.lev[m]] == g.full[P.lev[m]]) always += g.budget[P.lev[m]];
   }
-  const long long most = resident_blocks(sms, 8);
+  const long long most = resident_solve_blocks(sms);
   P.res_max = 0;
   if (sweeps <= 0 || always > most) return false;
   const bool done = resident_launch<8>(k_resident_solve, blocks, sms, st, P, sweeps);

@@ -85,3 +85,19 @@ def test_partly_allocated_full_level_is_solved(fake):  # noqa: F811
     fake.launches()
     s.project()
     assert [n.split(":")[1] for n in fake.launches() if "k_cluster_solve" in n] == ["1-0"]
+
+
+@pytest.mark.parametrize("sms,blocks,solver", [(152, (32, 32, 38), "k_resident_solve"), (152, (33, 33, 36), "k_dense_pass"),
+                                               (148, (32, 32, 37), "k_resident_solve"), (148, (34, 34, 33), "k_dense_pass")])
+def test_full_levels_beyond_the_resident_solve_are_dense(fake, sms, blocks, solver):  # noqa: F811
+    """The resident solve holds 256 blocks per SM; a full level of one more goes
+    to the dense passes, whatever the number of SMs, and none to the general solve."""
+    from dcgrid_gb300 import Simulation
+    fake.sms(sms)
+    x, y, z = blocks
+    s = Simulation(scenarios.plume(4 * x, 4 * y, 4 * z, x * y * z, 1, 4))
+    fake.launches()
+    s.project()
+    names = fake.launches()
+    used = {k for k in ("k_resident_solve", "k_dense_pass", "k_level_solve_batch") if any(k in n for n in names)}
+    assert used == {solver}
