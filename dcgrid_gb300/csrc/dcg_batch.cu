@@ -179,17 +179,18 @@ struct dcg_batch {
   }
   // the cascade with the tuned schedule of each round of the general solve
   void solve_tuned() {
-    solve([&](int round, int &grid, int &cache) {
+    cascade([&](SolveBatch &P, int round) {
+      if (launch_resident_solve(P, iters, sms, stream)) return;
       if (round < 4 && tune.round_ctas_per_sm[round] != 0) {
-        cache = tune.round_cache[round];
-        grid = batch_solve_grid(sms, cache, tune.round_ctas_per_sm[round]);
+        const int cache = tune.round_cache[round];
+        launch_level_solve_batch(P, iters, batch_solve_grid(sms, cache, tune.round_ctas_per_sm[round]), cache, stream);
       } else {
-        grid = solve_grid;
-        cache = tune.solve_cache;
+        launch_level_solve_batch(P, iters, solve_grid, tune.solve_cache, stream);
       }
     });
   }
-  template <class Schedule> void solve(Schedule schedule) {
+  // general(P, round): the levels that neither a cluster nor the dense passes take
+  template <class General> void cascade(General general) {
     std::vector<Dev> d(n());
     std::vector<char> raster(n());
     for (int i = 0; i < n(); i++) {
@@ -207,8 +208,6 @@ struct dcg_batch {
     c.sweeps = iters;
     c.st = stream;
     c.run(d.data(), raster.data(), n(), [&](const std::vector<int> &mem, const std::vector<int> &lev, long long limit, int round) {
-      int grid = 0, cache = 0;
-      schedule(round, grid, cache);
       for (size_t g = 0; g < mem.size(); g += BMAX) {
         SolveBatch P{};
         P.n = (int)std::min<size_t>(BMAX, mem.size() - g);
@@ -225,7 +224,7 @@ struct dcg_batch {
           P.lev[i] = lev[g + i];
           P.cl_max[i] = limit;
         }
-        if (!launch_resident_solve(P, iters, sms, stream)) launch_level_solve_batch(P, iters, grid, cache, stream);
+        general(P, round);
       }
     });
   }
@@ -444,31 +443,53 @@ struct dcg_batch {
       best.tile[stage] = tune.tile[stage] = tile_of[pick][stage];
       best.cells_ms[stage] = ms_of[pick][stage];
     }
-    // the general level solve (levels that no cluster holds): cache depth x
-    // CTAs per SM, timed with the whole cascade
-    float best_solve = 1e30f;
+    // the general level solve: cache depth x CTAs per SM, timed on the levels
+    // that may come to it as blocks are allocated, without the resident solve,
+    // which takes them until then. (Timed with the whole cascade, where it is
+    // mostly an empty launch, two runs on one batch chose variant 35 with three
+    // CTAs per SM and variant 8 with one.) Where no such level has a block for
+    // it there is nothing to time: the single simulations' variant, the best one
+    // just beyond the resident solve (ms per cascade of 100 sweeps, variants 19,
+    // 35, 83, 4: four levels of 12000 blocks 1.37, 1.41, 1.45, 1.58; one of 46601
+    // 1.29, 1.33, 1.40, 1.54; two of 100000 5.77, 5.81, 4.89, 6.48).
+    std::vector<SolveBatch> general;
+    cascade([&](SolveBatch &P, int) {
+      if (launch_resident_solve(P, iters, sms, stream)) return;
+      P.res_max = 0;
+      general.push_back(P);
+    });
+    if ((rc = sync())) return rc;
+    long long blocks = 0;
+    for (const SolveBatch &P : general)
+      for (int i = 0; i < P.n; i++) {
+        long long load = 0;
+        if ((rc = cuda(cudaMemcpy(&load, P.d[i].load + P.lev[i], sizeof(load), cudaMemcpyDeviceToHost), "load"))) return rc;
+        if (load > P.cl_max[i]) blocks += load;
+      }
     for (int r = 0; r < 4; r++) best.round_ctas_per_sm[r] = 0;
-    for (int cache : {0, 3, 4, 8, 16, 18, 19, 32, 34, 35, 64, 66, 83}) {
-      const int occ = batch_solve_grid(sms, cache, 0) / std::max(1, sms);
-      for (int k = 1; k <= occ; k++) {
-        const int grid = batch_solve_grid(sms, cache, k);
-        const float ms = time_ms(reps, [&] {
-          solve([&](int, int &g, int &c) {
-            g = grid;
-            c = cache;
+    best.solve_cache = dcg_sim::kSolveVariant;
+    best.solve_ctas_per_sm = 0;
+    if (blocks > 0) {
+      float best_solve = 1e30f;
+      for (int cache : {0, 3, 4, 8, 16, 18, 19, 32, 34, 35, 64, 66, 83}) {
+        const int occ = batch_solve_grid(sms, cache, 0) / std::max(1, sms);
+        for (int k = 1; k <= occ; k++) {
+          const int grid = batch_solve_grid(sms, cache, k);
+          const float ms = time_ms(reps, [&] {
+            for (const SolveBatch &P : general) launch_level_solve_batch(P, iters, grid, cache, stream);
           });
-        });
-        if (ms < best_solve) {
-          best_solve = ms;
-          best.solve_cache = cache;
-          best.solve_ctas_per_sm = k;
+          if (ms < best_solve) {
+            best_solve = ms;
+            best.solve_cache = cache;
+            best.solve_ctas_per_sm = k;
+          }
         }
       }
     }
-    best.solve_ms = best_solve;
-    if ((rc = sync())) return rc;
     tune = best;
     if ((rc = set_solve_config())) return rc;
+    tune.solve_ms = time_ms(reps, [&] { solve_tuned(); });
+    if ((rc = sync())) return rc;
     drop_graphs();
     if ((rc = reset())) return rc;
     if (out) *out = tune;

@@ -386,9 +386,10 @@ int dcg_batch_sync(dcg_batch *batch);      /* stream sync + every member's devic
 int dcg_batch_member(dcg_batch *batch, int32_t i, dcg_sim **out);
 int dcg_batch_set_stream(dcg_batch *batch, void *cuda_stream);
 /* Autotuner: resets the batch, runs spinup_steps steps, times every candidate
- * tile and solve schedule `reps` times with CUDA events, keeps the fastest,
- * and resets the batch again (the state is that of dcg_batch_reset after it;
- * results do not depend on the tuning). */
+ * tile `reps` times with CUDA events, and every candidate solve schedule on the
+ * levels that may come to the cooperative solve (variant 19 where none has a
+ * block for it), keeps the fastest, and resets the batch again (the state is
+ * that of dcg_batch_reset after it; results do not depend on the tuning). */
 int dcg_batch_autotune(dcg_batch *batch, int32_t spinup_steps, int32_t reps, dcg_tuning *out);
 int dcg_batch_get_tuning(const dcg_batch *batch, dcg_tuning *out);
 int dcg_batch_set_tuning(dcg_batch *batch, const dcg_tuning *tuning);

@@ -31,6 +31,7 @@ std::string g_log;
 std::vector<std::string> *g_capture = nullptr;
 cudaError_t g_last = cudaSuccess;
 int g_device = 0, g_sms = 152, g_raster_bad = 0;
+long long g_load = -1;
 double g_clock = 0;
 
 cudaError_t fail(cudaError_t e) {
@@ -104,6 +105,7 @@ cudaError_t copy(void *dst, const void *src, size_t n) {
   size_t left = 0;
   if ((block_of(dst, &left) && left < n) || (block_of(src, &left) && left < n)) return fail(cudaErrorInvalidValue);
   std::memcpy(dst, src, n);
+  if (g_load >= 0 && n == sizeof g_load && block_of(src, &left)) std::memcpy(dst, &g_load, n);
   return cudaSuccess;
 }
 cudaError_t fill(void *dst, int v, size_t n) {
@@ -125,6 +127,7 @@ void fake_refuse(const char *part) {  // launches of kernels with this in their 
 void fake_cost(const char *part, double ms) { g_cost[part] = ms; }
 void fake_sms(int n) { g_sms = n; }
 void fake_raster_bad(int bad) { g_raster_bad = bad; }
+void fake_load(long long blocks) { g_load = blocks; }  // what a read of one level's load gives; -1: what is there
 
 // ---------------------------------------------------------------- the runtime
 cudaError_t cudaGetLastError(void) {

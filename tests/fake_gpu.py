@@ -35,6 +35,9 @@ class Fake:
     def raster_bad(self, bad):
         self.lib.fake_raster_bad(int(bad))
 
+    def load(self, blocks):
+        self.lib.fake_load(C.c_longlong(blocks))
+
     def malloc(self, n):
         p = C.c_void_p()
         self.lib.cudaMalloc(C.byref(p), n)

@@ -101,3 +101,32 @@ def test_full_levels_beyond_the_resident_solve_are_dense(fake, sms, blocks, solv
     names = fake.launches()
     used = {k for k in ("k_resident_solve", "k_dense_pass", "k_level_solve_batch") if any(k in n for n in names)}
     assert used == {solver}
+
+
+def test_autotune_does_not_rank_a_general_solve_without_work(fake):  # noqa: F811
+    """Levels that the clusters hold never reach the general solve: its variants
+    have nothing to do, and their times would be noise."""
+    from dcgrid_gb300 import Batch
+    fake.cost("k_level_solve_batchILi8E", 1e-6)
+    fake.cost("k_cluster_solve", 0.05)
+    b = Batch(scenarios.plume_batch(3, 17, sizes=(16, 32), iters=10))
+    fake.launches()
+    t = b.autotune(spinup_steps=0, reps=1)
+    assert not any("k_level_solve_batch" in n for n in fake.launches())
+    assert (t["solve_cache"], t["solve_ctas_per_sm"]) == (19, 0)
+    assert t["solve_ms"] == pytest.approx(0.05)
+
+
+def test_autotune_times_the_general_solve_itself(fake):  # noqa: F811
+    """Levels that the resident solve takes while few of their blocks are
+    allocated, and the general solve afterwards: the latter is timed with work,
+    the cheapest of its variants chosen."""
+    from dcgrid_gb300 import Batch
+    fake.cost("k_level_solve_batch", 1.0)
+    fake.cost("k_level_solve_batchILi2ELi3E", 0.5)  # variant 34
+    fake.load(30000)
+    b = Batch([scenarios.plume(160, 160, 128, 6400 + 46601, 2, 4)])
+    fake.launches()
+    t = b.autotune(spinup_steps=1, reps=1)
+    timed = [n for n in fake.launches() if "k_level_solve_batch" in n and n.endswith("<0")]
+    assert t["solve_cache"] == 34 and len(timed) > 13
