@@ -7,6 +7,8 @@
 // reference's stage order. Differences: no exit(), status codes instead;
 // no host round trips inside a step; every launch goes to the handle's
 // stream, and dcg_step replays a captured CUDA graph of the whole step.
+#include <cuda.h>
+
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
@@ -316,6 +318,24 @@ static size_t field_cells(dcg_sim *s) {
   return s->mode == DCG_MODE_ADAPTIVE ? (size_t)s->D.g.B * BV : (size_t)s->U.nc;
 }
 
+// Whether a kernel may write `bytes` at dst where a copy did: memory of the
+// handle's GPU, aligned for floats and inside one allocation. A copy takes any
+// address, and refuses one that runs past its allocation; a kernel would fault.
+static bool kernel_target(const dcg_sim *s, const float *dst, size_t bytes) {
+  cudaPointerAttributes at{};
+  if (((uintptr_t)dst & 3) != 0 || cudaPointerGetAttributes(&at, dst) != cudaSuccess ||
+      at.type != cudaMemoryTypeDevice || at.device != s->device)
+    return false;
+  void *range = nullptr;
+  if (cudaGetDriverEntryPointByVersion("cuMemGetAddressRange", &range, 12000, cudaEnableDefault, nullptr) != cudaSuccess ||
+      !range)
+    return false;
+  CUdeviceptr base = 0;
+  size_t size = 0;
+  const CUdeviceptr p = (CUdeviceptr)(uintptr_t)dst;
+  return reinterpret_cast<decltype(&cuMemGetAddressRange)>(range)(&base, &size, p) == CUDA_SUCCESS &&
+         p - base <= size && bytes <= size - (size_t)(p - base);
+}
 int dcg_get_field(dcg_sim *s, int32_t field, float *dst, int32_t where) {
   if (bad(s) || !dst) return DCG_E_INVALID;
   const FieldRef r = field_ref(s, field);
@@ -323,10 +343,8 @@ int dcg_get_field(dcg_sim *s, int32_t field, float *dst, int32_t where) {
   const size_t cells = field_cells(s), n = cells * sizeof(float);
   int rc;
   const float *src = static_cast<const float *>(r.p);
-  if (r.mode) {  // 16-bit storage: widen into the buffer when it is this GPU's own memory, else into an FP32 staging buffer
-    cudaPointerAttributes at{};
-    if (where == DCG_DEVICE && cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
-        at.device == s->device) {
+  if (r.mode) {  // 16-bit storage: widen into the buffer where a kernel may, else into an FP32 staging buffer
+    if (where == DCG_DEVICE && kernel_target(s, dst, n)) {
       launch_h16_to_f32(static_cast<const uint16_t *>(r.p), dst, (long long)cells, r.mode, s->stream);
       if ((rc = s->check_launch("get_field"))) return rc;
       return s->sync("get_field");

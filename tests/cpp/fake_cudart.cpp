@@ -7,6 +7,7 @@
 // dynamic shared memory needs the opt-in of that kernel on the current device,
 // a refused launch leaves its error behind and no node in a graph under
 // capture, and a copy may not run past its allocation.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cstdlib>
@@ -177,6 +178,19 @@ cudaError_t cudaPointerGetAttributes(struct cudaPointerAttributes *a, const void
   std::memset(a, 0, sizeof *a);
   a->type = b ? cudaMemoryTypeDevice : cudaMemoryTypeUnregistered;
   a->device = b ? b->device : -1;
+  return cudaSuccess;
+}
+static CUresult address_range(CUdeviceptr *base, size_t *size, CUdeviceptr p) {
+  size_t left;
+  const Block *b = block_of(reinterpret_cast<const void *>(p), &left);
+  if (!b) return CUDA_ERROR_NOT_FOUND;
+  *base = p + left - b->bytes;
+  *size = b->bytes;
+  return CUDA_SUCCESS;
+}
+cudaError_t cudaGetDriverEntryPointByVersion(const char *symbol, void **f, unsigned, unsigned long long,
+                                             enum cudaDriverEntryPointQueryResult *) {
+  *f = std::strcmp(symbol, "cuMemGetAddressRange") ? nullptr : reinterpret_cast<void *>(address_range);
   return cudaSuccess;
 }
 cudaError_t cudaGetSymbolAddress(void **p, const void *s) {

@@ -130,3 +130,33 @@ def test_autotune_times_the_general_solve_itself(fake):  # noqa: F811
     t = b.autotune(spinup_steps=1, reps=1)
     timed = [n for n in fake.launches() if "k_level_solve_batch" in n and n.endswith("<0")]
     assert t["solve_cache"] == 34 and len(timed) > 13
+
+
+def test_kernels_write_only_buffers_that_a_copy_would_take(fake):  # noqa: F811
+    """A 16-bit field widens straight into an aligned buffer of the handle's GPU
+    that holds all of it. Anything else goes through a copy, which takes any
+    address and refuses one that runs past its allocation."""
+    import ctypes as C
+    from dcgrid_gb300 import Simulation
+    p = small_scene()
+    p.precision = capi.PRECISION_MIXED_FP16
+    s = Simulation(p)
+    n = 4 * s.num_cells
+
+    def into(buffer, offset=0):
+        """(status, whether a copy wrote the buffer); the kernels do nothing here"""
+        C.memset(buffer, 7, n // 2)
+        rc = s.L.dcg_get_field(s.h, capi.FIELD_NAMES["density"], C.c_void_p(buffer + offset), capi.DEVICE)
+        return rc, C.string_at(buffer + offset, n // 2 - offset) != b"\7" * (n // 2 - offset)
+    own = fake.malloc(n + 8)
+    assert into(own) == (capi.DCG_OK, False)
+    assert into(own, 4) == (capi.DCG_OK, False)
+    assert into(own, 2) == (capi.DCG_OK, True)
+    small = fake.malloc(n // 2)
+    fake.malloc(n)
+    assert into(small) == (capi.DCG_E_CUDA, False)
+    fake.lib.cudaGetLastError()
+    fake.device(1)
+    other = fake.malloc(n)
+    fake.device(0)
+    assert into(other) == (capi.DCG_OK, True)
