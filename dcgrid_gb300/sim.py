@@ -152,8 +152,10 @@ def _buf(obj, count, dtype, what, writable=False, device=False):
 
 def _produced(obj, sim):
     """Waits for torch's current stream when `obj` is a CUDA tensor and that
-    stream is not the handle's: the library reads the tensor on the handle's
-    stream, which is not ordered behind the one that computes it."""
+    stream is not the handle's: the library reads the tensor (and any other of
+    the same call) on the handle's stream, which is not ordered behind the one
+    that computes it. Calls that only write a tensor do not wait (3 us): what
+    torch still has queued on it is the caller's to finish first."""
     if getattr(obj, "is_cuda", False):
         import torch
         stream = torch.cuda.current_stream(obj.device)
@@ -250,8 +252,8 @@ class Simulation:
         if n == 0:  # no emission map: the library reports it
             self._chk(self.L.dcg_set_emission(self.h, _ptr(np.zeros(1, np.float32)), capi.HOST), "set_emission")
         ptr, where = _buf(a, n, np.float32, "set_emission")
-        if where == capi.HOST:
-            self._emis_keep = a  # an asynchronous copy may still read it
+        self._emis_keep = a  # an asynchronous copy may still read it
+        _produced(a, self)
         self._chk(self.L.dcg_set_emission(self.h, ptr, where), "set_emission")
 
     def set_heightmap(self, heights):
@@ -418,6 +420,7 @@ class Simulation:
         if lam_emission is not None and self.params.emission_n > 0:
             em, _ = _buf(lam_emission, int(self.params.emission_n) ** 3, np.float32, "adjoint_step lam_emission",
                          device=True)
+        _produced(lam_in, self)
         self._chk(self.L.dcg_adjoint_step(self.h, li, lo, em), "adjoint_step")
 
     def adjoint_step_full(self, lam_in, lam_out, lam_emission=None):
@@ -433,12 +436,14 @@ class Simulation:
         if lam_emission is not None and self.params.emission_n > 0:
             em, _ = _buf(lam_emission, int(self.params.emission_n) ** 3, np.float32,
                          "adjoint_step_full lam_emission", device=True)
+        _produced(lam_in, self)
         self._chk(self.L.dcg_adjoint_step_full(self.h, li, lo, em), "adjoint_step_full")
 
     def adjoint_dense(self, lam_dense, lam_cells):
         p = self.params
         ld, _ = _buf(lam_dense, p.gx * p.gy * p.gz, np.float32, "adjoint_dense lam_dense", device=True)
         lc, _ = _buf(lam_cells, self.num_cells, np.float32, "adjoint_dense lam_cells", device=True)
+        _produced(lam_dense, self)
         self._chk(self.L.dcg_adjoint_dense(self.h, ld, lc), "adjoint_dense")
 
     def stats(self):
@@ -626,6 +631,8 @@ class Batch:
 
     def set_stream(self, stream_ptr):
         self._chk(self.L.dcg_batch_set_stream(self.h, C.c_void_p(stream_ptr)), "set_stream")
+        for h in [self] + self.members:
+            h._stream_ptr = stream_ptr
 
     def autotune(self, spinup_steps=10, reps=3):
         t = capi.DcgTuning()
@@ -655,8 +662,8 @@ class Batch:
             self._chk(self.L.dcg_batch_set_emission(self.h, _ptr(np.zeros(1, np.float32)), capi.HOST),
                       "set_emission")
         ptr, where = _buf(a, n, np.float32, "set_emission")
-        if where == capi.HOST:
-            self._emis_keep = a  # an asynchronous copy may still read it
+        self._emis_keep = a  # an asynchronous copy may still read it
+        _produced(a, self)
         self._chk(self.L.dcg_batch_set_emission(self.h, ptr, where), "set_emission")
 
     def stats(self):

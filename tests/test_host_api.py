@@ -169,3 +169,83 @@ def test_reference_named_classes_have_the_reference_methods():
                "render", "debugStats"]
     for cls in (sim.FluidSimulationDCGrid, sim.FluidSimulationUniform):
         assert all(callable(getattr(cls, m, None)) for m in methods), cls
+
+
+class CudaTensor:
+    """What the host layer reads of a float32 CUDA tensor."""
+    is_cuda, dtype, device = True, "torch.float32", "cuda:0"
+
+    def __init__(self, n):
+        self.shape = (n,)
+
+    def data_ptr(self):
+        return 4096
+
+    def is_contiguous(self):
+        return True
+
+    def numel(self):
+        return self.shape[0]
+
+
+def fake_batch():
+    from dcgrid_gb300 import sim
+    b = object.__new__(sim.Batch)
+    b.L, b.h, b.members = FakeLib(), C.c_void_p(1), []
+    b.params = [capi.default_params(16, 16, 16, 50)]
+    b.params[0].emission_n = 4
+    return b
+
+
+# every call that reads CUDA tensors: (handle, call)
+READS = {
+    "set_field": (fake_sim, lambda s: s.set_field("density", CudaTensor(s.num_cells))),
+    "set_emission": (fake_sim, lambda s: s.set_emission(CudaTensor(64))),
+    "batch set_emission": (fake_batch, lambda b: b.set_emission(CudaTensor(64))),
+    "adjoint_step": (fake_sim, lambda s: s.adjoint_step(CudaTensor(s.num_cells), CudaTensor(s.num_cells), CudaTensor(64))),
+    "adjoint_step_full": (fake_sim, lambda s: s.adjoint_step_full(CudaTensor(4 * s.num_cells),
+                                                                  CudaTensor(4 * s.num_cells), CudaTensor(64))),
+    "adjoint_dense": (fake_sim, lambda s: s.adjoint_dense(CudaTensor(16 * 32 * 16), CudaTensor(s.num_cells))),
+}
+
+
+@pytest.mark.parametrize("own_stream", [True, False])
+@pytest.mark.parametrize("name", READS)
+def test_tensors_are_read_after_their_stream(name, own_stream, monkeypatch):
+    """torch's current stream computes a tensor, the handle's stream reads it: the
+    call waits unless they are one stream."""
+    torch = pytest.importorskip("torch")
+    make, call = READS[name]
+    h = make()
+
+    class Stream:
+        cuda_stream = 77
+
+        def synchronize(self):
+            h.L.calls.append(("synchronize", ()))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
+    h.set_stream(88 if own_stream else 77)
+    h.L.calls.clear()
+    call(h)
+    assert h.L.names() == (["synchronize"] if own_stream else []) + [h.L.names()[-1]]
+    assert h.L.names()[-1].startswith("dcg_")
+
+
+@pytest.mark.parametrize("make", [fake_sim, fake_batch])
+def test_emission_tensors_outlive_their_copy(make, monkeypatch):
+    """The copy is asynchronous: the handle keeps the tensor until the next map."""
+    import weakref
+    torch = pytest.importorskip("torch")
+    h = make()
+
+    class Stream:
+        cuda_stream = 77
+
+        def synchronize(self):
+            pass
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
+    t = CudaTensor(64)
+    kept = weakref.ref(t)
+    h.set_emission(t)
+    del t
+    assert kept() is not None
