@@ -667,9 +667,14 @@ int dcg_render(dcg_sim *s, const dcg_render_params *rp, float *rgba, int32_t whe
   if (s->mode == DCG_MODE_ADAPTIVE) {
     // the frame's scratch is kept for the next one: its size is the handle's
     const size_t need = render_scratch_bytes(s->D.g, R);
-    if (need && !s->render_scratch && cudaMalloc(&s->render_scratch, need) != cudaSuccess) {
-      cudaGetLastError();
-      s->render_scratch = nullptr;
+    if (need && !s->render_scratch) {
+      if (cudaMalloc(&s->render_scratch, need) == cudaSuccess) {
+        s->allocs.push_back(s->render_scratch);
+        s->bytes += need;
+      } else {  // the frame walks the tree instead
+        cudaGetLastError();
+        s->render_scratch = nullptr;
+      }
     }
     if (need && s->render_scratch) launch_render_tiled(s->D, R, s->render_scratch, out, s->stream);
     else launch_render_adaptive(s->D, R, out, s->stream);

@@ -230,7 +230,6 @@ struct dcg_sim {
   }
   ~dcg_sim() {
     if (render_tmp) cudaFree(render_tmp);
-    if (render_scratch) cudaFree(render_scratch);
     if (hmap) cudaFree(hmap);
     free_all();
     if (own_stream && stream) cudaStreamDestroy(stream);

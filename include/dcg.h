@@ -442,6 +442,9 @@ typedef struct {
  * (src/simulation.cpp:153-156: Fluid, 1, on, on; defaultParams' Resolution
  * channel is overwritten every frame); eye outside the domain looking along +z */
 void dcg_default_render_params(dcg_render_params *rp, int32_t width, int32_t height);
+/* The first frame of the fluid channel of an adaptive handle of up to 2^18
+ * blocks allocates 865 bytes per block and 4 per finest block of the domain,
+ * kept and counted in dcg_info.device_bytes; refused, the frames take longer. */
 int dcg_render(dcg_sim *sim, const dcg_render_params *rp, float *rgba, int32_t where);
 
 /* ---- memory-budget calculator (the reference's scripts/calcMemory*.js,

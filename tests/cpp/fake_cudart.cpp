@@ -126,6 +126,11 @@ void fake_refuse(const char *part) {  // launches of kernels with this in their 
   if (*part) g_refused.insert(part);
 }
 void fake_cost(const char *part, double ms) { g_cost[part] = ms; }
+long long fake_held(void) {  // bytes allocated
+  long long n = 0;
+  for (auto &b : g_mem) n += (long long)b.second.bytes;
+  return n;
+}
 void fake_sms(int n) { g_sms = n; }
 void fake_raster_bad(int bad) { g_raster_bad = bad; }
 void fake_load(long long blocks) { g_load = blocks; }  // what a read of one level's load gives; -1: what is there

@@ -18,6 +18,7 @@ class Fake:
         self.lib = lib
         lib.fake_log.restype = C.c_char_p
         lib.fake_cost.argtypes = [C.c_char_p, C.c_double]
+        lib.fake_held.restype = C.c_longlong
         lib.cudaMalloc.argtypes = [C.POINTER(C.c_void_p), C.c_size_t]
 
     def device(self, d):
@@ -37,6 +38,9 @@ class Fake:
 
     def load(self, blocks):
         self.lib.fake_load(C.c_longlong(blocks))
+
+    def held(self):
+        return self.lib.fake_held()
 
     def malloc(self, n):
         p = C.c_void_p()

@@ -160,3 +160,24 @@ def test_kernels_write_only_buffers_that_a_copy_would_take(fake):  # noqa: F811
     other = fake.malloc(n)
     fake.device(0)
     assert into(other) == (capi.DCG_OK, True)
+
+
+def test_frame_scratch_is_counted(fake):  # noqa: F811
+    """device_bytes is the memory that the handle holds, a frame's tiles and map
+    (allocated by the first frame) included; none of it is left behind."""
+    import ctypes as C
+    from dcgrid_gb300 import Simulation
+    from dcgrid_gb300.sim import default_render_params
+    held = fake.held()
+    p = small_scene()
+    s = Simulation(p)
+    before = s.info.device_bytes
+    assert fake.held() - held == before
+    rp = default_render_params(8, 8, p)
+    image = fake.malloc(8 * 8 * 16)
+    for _ in range(2):
+        assert s.L.dcg_render(s.h, C.byref(rp), C.c_void_p(image), capi.DEVICE) == capi.DCG_OK
+        s.L.dcg_get_info(s.h, C.byref(s.info))
+        assert s.info.device_bytes == fake.held() - held - 8 * 8 * 16 > before
+    s.close()
+    assert fake.held() - held == 8 * 8 * 16
