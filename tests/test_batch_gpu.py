@@ -254,3 +254,28 @@ def test_batch_emission_upload_equals_member_uploads():
         s.sync()
     for i, p in enumerate(params):
         compare(a[i], b[i], p, f"member {i}")
+
+
+def test_every_variant_of_the_general_solve():
+    """Two members whose sparse levels meet in one launch (level 0 of one, level 1
+    of the other) with more allocated blocks than the resident solve holds: each
+    variant of the general solve, which takes them, gives the standalone results."""
+    import torch
+    from dcgrid_gb300 import Batch
+    params = [scenarios.plume(160, 160, 128, 20 * 20 * 16 + 46601, 2, 4),
+              scenarios.plume(176, 176, 144, 11 * 11 * 9 + 6000, 3, 4)]
+    ref = [standalone(p, 2) for p in params]
+    limit = 256 * torch.cuda.get_device_properties(0).multi_processor_count
+    loads = [s.get_topology()["load"] for s in ref]
+    assert loads[0][0] > limit and loads[1][1] > 1024 and ref[1].info.full_blocks[2] > 1024
+    b = Batch(params)
+    for cache in (0, 3, 4, 8, 16, 18, 19, 32, 34, 35, 64, 66, 83):
+        for ctas in (0, 1):
+            b.set_tuning(tuning(1, cache, ctas, 1, 1))
+            b.reset()
+            for m in b:
+                m.add_velocity_noise(11, 0.05)
+            b.step(2)
+            b.sync()
+            for i, p in enumerate(params):
+                compare(b[i], ref[i], p, f"variant {cache}, {ctas} CTAs per SM, member {i}")

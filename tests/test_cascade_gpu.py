@@ -255,3 +255,55 @@ def test_tiles_beyond_the_box_cost_no_division_tests():
         s.close()
     print("us per sweep:", [round(10 * t, 2) for t in best])
     assert best[0] < 1.25 * best[1]
+
+
+def test_blocks_out_of_raster_order_leave_the_dense_passes():
+    """A state whose full level (39936 blocks, the dense passes') lists its blocks
+    in another order: the order is noticed, and the projection gives the same
+    pressures and velocities, block for block."""
+    from dcgrid_gb300 import Simulation
+    p = scenarios.plume(256, 256, 312, 32 * 32 * 39 + 300, 2, 4)
+    a, b = Simulation(p), Simulation(p)
+    a.add_velocity_noise(5, 0.5)
+    a.step(1)
+    state = a.save_state()
+    B, nc = p.max_blocks, 64 * p.max_blocks
+    off, full = int(a.info.offset[1]), int(a.info.full_blocks[1])
+    to = np.arange(B)
+    to[off:off + full] = off + np.random.default_rng(4).permutation(full)
+    none = np.uint32(0xFFFFFFFF)
+    at = 64  # the header
+
+    def section(count, dtype):
+        nonlocal at
+        s = moved[at:at + count * np.dtype(dtype).itemsize].view(dtype)
+        at += s.nbytes
+        return s
+
+    def reorder(s, per_block):
+        v = s.reshape(B, per_block)
+        v[to] = v.copy()
+
+    moved = state.copy()
+    reorder(section(4 * B, np.int32), 4)  # pos
+    for per_block, low in ((1, 3), (8, 0), (27, 0)):  # parent, child, neighbours; subblock bits
+        s = section(per_block * B, np.uint32)
+        known = s != none
+        high = s[known] & np.uint32(0xF0000000) if per_block == 27 else np.uint32(0)
+        e = s[known] & np.uint32(0x0FFFFFFF) if per_block == 27 else s[known]
+        s[known] = high | (to[e >> low].astype(np.uint32) << low) | (e & np.uint32((1 << low) - 1))
+        reorder(s, per_block)
+    reorder(section(B, np.uint8), 1)  # flags
+    section(32, np.int64)             # loads and move limits
+    while at < len(moved):
+        reorder(section(nc, np.float32), 64)
+    assert at == len(moved)
+    b.load_state(moved)
+    for s in (a, b):
+        s.project()
+        s.sync()
+    cells = (64 * to[:, None] + np.arange(64)).reshape(-1)
+    alloc = np.repeat(a.get_topology()["pos"][:, 3] >= 0, 64)
+    for f in ("pressure", "divergence", "vel_x", "vel_y", "vel_z"):
+        x, y = a.get_field(f), b.get_field(f)[cells]
+        assert np.array_equal(x[alloc].view(np.uint32), y[alloc].view(np.uint32)), f
