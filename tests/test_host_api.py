@@ -173,7 +173,10 @@ def test_reference_named_classes_have_the_reference_methods():
 
 class CudaTensor:
     """What the host layer reads of a float32 CUDA tensor."""
-    is_cuda, dtype, device = True, "torch.float32", "cuda:0"
+    is_cuda, dtype = True, "torch.float32"
+
+    class device:
+        index = 0
 
     def __init__(self, n):
         self.shape = (n,)
@@ -197,6 +200,20 @@ def fake_batch():
     return b
 
 
+@pytest.fixture
+def torch_stream(monkeypatch):
+    """torch's current stream is number 77; sync[0] is called when it is waited for"""
+    torch = pytest.importorskip("torch")
+    sync = [lambda: None]
+
+    class Stream:
+        def synchronize(self):
+            sync[0]()
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 77, raising=False)
+    return sync
+
+
 # every call that reads CUDA tensors: (handle, call)
 READS = {
     "set_field": (fake_sim, lambda s: s.set_field("density", CudaTensor(s.num_cells))),
@@ -211,19 +228,12 @@ READS = {
 
 @pytest.mark.parametrize("own_stream", [True, False])
 @pytest.mark.parametrize("name", READS)
-def test_tensors_are_read_after_their_stream(name, own_stream, monkeypatch):
+def test_tensors_are_read_after_their_stream(name, own_stream, torch_stream):
     """torch's current stream computes a tensor, the handle's stream reads it: the
     call waits unless they are one stream."""
-    torch = pytest.importorskip("torch")
     make, call = READS[name]
     h = make()
-
-    class Stream:
-        cuda_stream = 77
-
-        def synchronize(self):
-            h.L.calls.append(("synchronize", ()))
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
+    torch_stream[0] = lambda: h.L.calls.append(("synchronize", ()))
     h.set_stream(88 if own_stream else 77)
     h.L.calls.clear()
     call(h)
@@ -232,18 +242,10 @@ def test_tensors_are_read_after_their_stream(name, own_stream, monkeypatch):
 
 
 @pytest.mark.parametrize("make", [fake_sim, fake_batch])
-def test_emission_tensors_outlive_their_copy(make, monkeypatch):
+def test_emission_tensors_outlive_their_copy(make, torch_stream):
     """The copy is asynchronous: the handle keeps the tensor until the next map."""
     import weakref
-    torch = pytest.importorskip("torch")
     h = make()
-
-    class Stream:
-        cuda_stream = 77
-
-        def synchronize(self):
-            pass
-    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: Stream())
     t = CudaTensor(64)
     kept = weakref.ref(t)
     h.set_emission(t)
