@@ -601,13 +601,13 @@ int dcg_check_div6(uint64_t *mismatches, uint32_t *first) {
 int dcg_check_barrier_timeout(dcg_sim *s, uint32_t poll_limit) {
   if (bad(s) || s->mode != DCG_MODE_ADAPTIVE || poll_limit == 0 || poll_limit > (1u << 20)) return DCG_E_INVALID;
   if (member_refused(s)) return DCG_E_INVALID;
-  const size_t bar_bytes = 4 * (64 + 32 * 18);
+  const size_t bar_bytes = sizeof(*s->D.bar);
   int rc;
   if ((rc = s->cuda(cudaMemsetAsync(s->D.bar, 0, bar_bytes, s->stream), "barrier check"))) return rc;
   if ((rc = s->cuda((cudaError_t)launch_barrier_probe(s->D.bar, s->D.err, poll_limit, 2, s->stream),
                     "barrier check launch")))
     return rc;
-  // the waiting CTA's arrival stays counted: clear the words for the next solve
+  // the waiting CTA's arrival stays counted: clear the word for the next solve
   return s->cuda(cudaMemsetAsync(s->D.bar, 0, bar_bytes, s->stream), "barrier check");
 }
 

@@ -7,13 +7,15 @@
 // over all members: the members' device descriptors travel in the kernel
 // parameters, and a CTA picks its member from the cumulative CTA counts.
 // The pressure cascade solves small levels of all members on chip, one cluster
-// per member (k_cascade.cu), larger ones by one cooperative launch over the
-// members' concatenated cells; p, p~ and div of all members are slices of
-// three batch arenas so that solve addresses them with one base pointer. The
-// adaptation (scores, radix sorts, selections, moves, refinements, neighbour
-// rebuild, propagation) is likewise one launch per adaptation kernel over all
-// members, each member's sorts and counters kept separate. Per-member arithmetic is the
-// single simulation's, so results are bit-identical to standalone runs.
+// per member (k_cascade.cu), large full ones in dense passes (k_dense.cu), the
+// others by cooperative launches over the members' concatenated blocks
+// (k_resident.cu, k_fluid.cu); p, p~ and div of all members are slices of three
+// batch arenas so that those address them with one base pointer. The adaptation
+// (scores, one CTA's decisions per member, rescoring, neighbour rebuild,
+// propagation; beyond 131072 blocks in a member the sequence with radix sorts)
+// is likewise one launch per adaptation kernel over all members, each member's
+// lists and counters kept separate. Per-member arithmetic is the single
+// simulation's, so results are bit-identical to standalone runs.
 #include <chrono>
 
 #include "dcg_sim.h"
@@ -353,7 +355,7 @@ struct dcg_batch {
   int reset() {
     int rc;
     if ((rc = cuda(cudaStreamSynchronize(stream), "sync"))) return rc;
-    cudaMemsetAsync(bar, 0, 4 * (64 + 32 * 18), stream);
+    cudaMemsetAsync(bar, 0, 4, stream);
     cudaMemsetAsync(errw, 0, 4, stream);
     for (dcg_sim *s : m)
       if ((rc = s->reset_adaptive())) return fail(rc, "member reset: " + s->err);
@@ -601,11 +603,11 @@ int dcg_batch_create(int32_t n, const dcg_params *params, dcg_batch **out) {
   }
   if ((rc = b->alloc(&b->p_arena, cells)) || (rc = b->alloc(&b->pt_arena, cells)) ||
       (rc = b->alloc(&b->div_arena, cells)) || (rc = b->alloc(&b->binfo, BI_WORDS * (cells / BV))) ||
-      (rc = b->alloc(&b->bar, 64 + 32 * 18)) || (rc = b->alloc(&b->errw, 4))) {
+      (rc = b->alloc(&b->bar, 1)) || (rc = b->alloc(&b->errw, 4))) {
     delete b;
     return rc;
   }
-  cudaMemset(b->bar, 0, 4 * (64 + 32 * 18));
+  cudaMemset(b->bar, 0, 4);
   for (int i = 0; i < n; i++)
     if (params[i].emission_n > 0)
       b->emis_floats += (size_t)params[i].emission_n * params[i].emission_n * params[i].emission_n;

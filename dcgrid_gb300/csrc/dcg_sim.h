@@ -176,13 +176,13 @@ struct dcg_sim {
   // the full levels are allocated in full and lie in raster order, as created (a
   // caller's topology or state may say otherwise: check_raster)
   char raster = 1;
-  // level solve of single simulations: pipelined staged sweeps, two tile buffers,
-  // block descriptions cached in 3 x 8 KB of shared memory when they fit.
-  // Variant 19 (3 CTAs per SM, two blocks per claim); variant 83 (4 CTAs per
-  // SM, one block per claim) measured faster on the 256^3 cloud (1.85 against
-  // 1.93 ms per step) but slower on the 16 plumes stepped as single
-  // simulations (27.3 against 26.5 ms) and on the reference-default scenes
-  // (2.01 / 4.00 against 1.99 / 3.89 ms per step).
+  // general solve of single simulations, which takes sparse levels that the
+  // resident solve cannot hold: pipelined staged sweeps, two tile buffers, block
+  // descriptions cached in 3 x 8 KB of shared memory when they fit, 3 CTAs per
+  // SM, two blocks per claim. Variant 83 (4 CTAs per SM, one block per claim) is
+  // slower just beyond that line and faster far from it (ms per cascade of 100
+  // sweeps, 19 and 83: 46601 blocks 1.29 and 1.40, two levels of 100000 blocks
+  // 5.77 and 4.89).
   static constexpr int kSolveVariant = 19;
   // batch members: p and p~ are slices of the batch's arenas, and the batch
   // steps the member (its own step and stage entry points are refused)
@@ -396,7 +396,7 @@ struct dcg_sim {
     if ((rc = alloc(&D.ctr, C_COUNT))) return rc;
     if ((rc = alloc(&D.err, 4))) return rc;
     if ((rc = alloc(&D.red, 32))) return rc;
-    if ((rc = alloc(&D.bar, 64 + 32 * 18))) return rc;
+    if ((rc = alloc(&D.bar, 1))) return rc;
     if ((rc = alloc(&D.binfo, (long long)BI_WORDS * B))) return rc;
     if (P.defect_passes > 0) {
       if (ext_rr) {
@@ -491,7 +491,7 @@ struct dcg_sim {
     cudaMemsetAsync(D.nbr, 0xff, (size_t)27 * D.g.B * 4, stream);
     cudaMemsetAsync(D.ctr, 0, sizeof(long long) * C_COUNT, stream);
     cudaMemsetAsync(D.err, 0, 4, stream);
-    cudaMemsetAsync(D.bar, 0, 4 * (64 + 32 * 18), stream);
+    cudaMemsetAsync(D.bar, 0, 4, stream);
     long long load[MAXL] = {0}, ml[MAXL] = {0};
     for (int l = 0; l < D.g.levels; l++) load[l] = D.g.budget[l] == D.g.full[l] ? D.g.budget[l] : 0;
     if ((rc = cuda(cudaMemcpyAsync(D.load, load, sizeof(load), cudaMemcpyHostToDevice, stream), "load"))) return rc;

@@ -36,11 +36,11 @@ namespace dcg {
 // The order of the sum is the layout's: an adaptive level marches along x (x,
 // y, z neighbours = M, B, A), the uniform grid along z (A, B, M).
 // What bounds it: the shared-memory pipe (about 46 wavefronts per warp, step
-// and sweep of 256 cells, 83 % of a step's cycles on a 512^3 box) and the
-// chain of T sweeps inside a step. T = 4 in 512 threads of 116 registers;
+// and sweep of 256 cells; L1 80 % busy over a pass of 256^3 cells, issue 31 %)
+// and the chain of T sweeps inside a step. T = 4 in 512 threads of 116 registers;
 // measured slower: T = 3 in 640 threads (17.8 against 15.1 ms for 100 sweeps
-// of 512^3), T = 2 in 768 (17.9), the planes before kept in registers for
-// every sweep (spills, 21 ms) or for three of four (15.6). Against one sweep
+// of 512^3; 14.7 now), T = 2 in 768 (17.9), the planes before kept in registers
+// for every sweep (spills, 21 ms) or for three of four (15.6). Against one sweep
 // per pass over memory (grid-wide cooperative solve, 3.3 TB/s): 48.7 ms.
 template <int T> __host__ __device__ constexpr int dn_threads() { return T == 2 ? 640 : 512; }
 template <int T> __host__ __device__ constexpr uint32_t dn_plane() { return dn_threads<T>() * 32; }  // bytes of a tile plane

@@ -1733,9 +1733,9 @@ void launch_check_div6(unsigned long long *bad, int sms, cudaStream_t st) {
 }
 
 // Self-check of the bounded grid-barrier wait: CTA `absent` leaves without
-// arriving, so the others wait on a generation word that nothing advances,
-// give up after `limit` polls and record DCG_DEVERR_TIMEOUT; the second
-// barrier must then return at once (the error bit short-cuts it).
+// arriving, so the others wait for a flip of the barrier's word that does not
+// come, give up after `limit` polls and record DCG_DEVERR_TIMEOUT; the second
+// barrier must then return at once (the error bit ends its wait).
 __global__ void __launch_bounds__(64) k_barrier_probe(uint32_t *bar, uint32_t *errw, unsigned limit,
                                                       unsigned absent) {
   if (blockIdx.x == absent) return;

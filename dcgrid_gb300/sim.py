@@ -572,8 +572,8 @@ class _Member(Simulation):
 
 class Batch:
     """Many independent adaptive simulations stepped together (dcg_batch_*):
-    one launch per field stage over all members, one cooperative launch per
-    cascade round, member adaptations as parallel graph branches."""
+    the launches of every stage, of the pressure solve and of the adaptation
+    cover all members, and the step is one graph."""
 
     def __init__(self, params_list):
         self.L = lib()

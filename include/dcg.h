@@ -335,12 +335,10 @@ int dcg_check_barrier_timeout(dcg_sim *sim, uint32_t poll_limit);
  * (one global __constant__ parameter set, src/utils/sim_utils.h:5-6). A batch
  * owns n adaptive simulations with their own parameters, domains, level
  * counts and budgets; every field stage of a batch step is one launch over
- * all members (groups of 16 members per launch), each cascade round of the
- * pressure solve is one cooperative launch over the members' cells, the
- * members' adaptations run as parallel branches, and the whole step is one
- * CUDA graph. A member's results equal those of a standalone simulation with
- * the same parameters, bit for bit. All members must use the same
- * jacobi_iters. */
+ * all members (groups of 16 members per launch), the pressure solve's launches
+ * and the adaptation's cover all members too, and the whole step is one CUDA
+ * graph. A member's results equal those of a standalone simulation with the
+ * same parameters, bit for bit. All members must use the same jacobi_iters. */
 typedef struct dcg_batch dcg_batch;
 typedef struct {
   int32_t tile[4];           /* blocks of 64 cells per CTA (2, 4 or 8) for advect velocity,
