@@ -435,7 +435,9 @@ template <int K, class Kernel, class... Args>
 static bool resident_launch(Kernel kernel, long long blocks, int sms, cudaStream_t st, const Args &...args) {
   const size_t smem = Rests<K>::kBytes;
   int occ = 0;
-  // a device that refuses the launch has the other solvers: no error is left behind
+  // a device that refuses the launch has the other solvers: no error is left
+  // behind, but one of an earlier launch is not cleared with it
+  if (cudaPeekAtLastError() != cudaSuccess) return false;
   auto ok = [](cudaError_t e) {
     if (e != cudaSuccess) cudaGetLastError();
     return e == cudaSuccess;

@@ -439,10 +439,11 @@ void launch_u_project(const UDev &U, int top_pairs, int pairs, bool local, bool 
     int l = top;
     while (l >= 0 && ucells(U, l) <= SB_CELLS) l--;
     if (l < top) {  // the levels that one CTA holds; the shared-memory opt-in is the current device's
+      const bool clean = cudaPeekAtLastError() == cudaSuccess;
       if (cudaFuncSetAttribute(k_u_small, cudaFuncAttributeMaxDynamicSharedMemorySize, SB_SMEM) == cudaSuccess) {
         k_u_small<<<1, SB_THREADS, SB_SMEM, st>>>(U, top, l + 1, 2 * top_pairs, 2 * pairs);
       } else {
-        cudaGetLastError();  // a launch per sweep takes its place
+        if (clean) cudaGetLastError();  // a launch per sweep takes its place
         l = top;
       }
     }

@@ -121,9 +121,9 @@ extern "C" {
 // ---------------------------------------------------------------- the tests' side
 const char *fake_log(void) { return g_log.c_str(); }  // launches since the last fake_clear, a name per line
 void fake_clear(void) { g_log.clear(); }
-void fake_refuse(const char *part) {  // launches of kernels with this in their name; "": none
-  g_refused.clear();
+void fake_refuse(const char *part) {  // launches of kernels with this in their name too; "": none
   if (*part) g_refused.insert(part);
+  else g_refused.clear();
 }
 void fake_cost(const char *part, double ms) { g_cost[part] = ms; }
 long long fake_held(void) {  // bytes allocated
@@ -136,6 +136,7 @@ void fake_raster_bad(int bad) { g_raster_bad = bad; }
 void fake_load(long long blocks) { g_load = blocks; }  // what a read of one level's load gives; -1: what is there
 
 // ---------------------------------------------------------------- the runtime
+cudaError_t cudaPeekAtLastError(void) { return g_last; }
 cudaError_t cudaGetLastError(void) {
   const cudaError_t e = g_last;
   g_last = cudaSuccess;

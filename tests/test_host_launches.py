@@ -181,3 +181,19 @@ def test_frame_scratch_is_counted(fake):  # noqa: F811
         assert s.info.device_bytes == fake.held() - held - 8 * 8 * 16 > before
     s.close()
     assert fake.held() - held == 8 * 8 * 16
+
+
+def test_a_solver_that_gives_way_hides_no_other_refusal(fake):  # noqa: F811
+    """The resident solve, when refused, leaves its levels to the general solve and
+    no error; an error that is there already stays."""
+    from dcgrid_gb300 import DcgError, Simulation
+    s = Simulation(scenarios.plume(64, 64, 64, 512 + 4000, 2, 4))
+    fake.refuse("k_resident_solve")
+    fake.launches()
+    s.step(2)
+    assert any("k_level_solve_batch" in n for n in fake.launches())
+    s = Simulation(scenarios.plume(64, 64, 64, 512 + 4000, 2, 4))
+    fake.refuse("k_decide")
+    for _ in range(2):
+        with pytest.raises(DcgError):
+            s.step(1)
